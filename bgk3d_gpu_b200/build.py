@@ -29,7 +29,7 @@ NVCC_FLAGS = ARCH + [
 ]
 
 LIB_SOURCES = ["bgk_api.cu", "lattice.cu", "lattice_io.cu", "diag.cu", "batch.cu", "noalloc.cu", "devmem.cu"] + [
-    f"inst_{kind}_{group}.cu" for kind in ("f64", "f32", "f16", "bf16", "f32f64") for group in ("ab", "aa", "batch", "misc")]
+    f"inst_{kind}_{group}.cu" for kind in ("f64", "f32", "f16", "bf16", "f32f64") for group in ("ab", "t2", "aa", "batch", "misc")]
 LIB = "libbgk3d_b200.so"
 DROPIN_SP = "libbgk3d_dropin_sp.so"
 DROPIN_DP = "libbgk3d_dropin_dp.so"

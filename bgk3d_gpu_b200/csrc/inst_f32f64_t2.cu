@@ -1,0 +1,3 @@
+// Kernel instantiations (two-lattice time step) for storage float, compute double.
+#include "launch.cuh"
+BGK_INSTANTIATE_T2(float, double)

@@ -15,6 +15,9 @@ template <class S, class C>
 int launch_sweep_tma(const bgk_sweep_params* p, void* const* a, void* const* b, const void* tmap, const int* pa,
                      int* err, cudaStream_t st);
 template <class S, class C>
+int launch_sweep_t2(const bgk_sweep_params* p, void* const* a, void* const* b, const uint32_t* links, int* err,
+                    bool outflow_fresh, cudaStream_t st);
+template <class S, class C>
 int launch_moments(const bgk_sweep_params* p, void* const* a, double* out, double* ws, cudaStream_t st);
 template <class S, class C>
 int launch_draglift(const bgk_sweep_params* p, void* const* a, int is, int ie, int js, int je, int ks, int ke,

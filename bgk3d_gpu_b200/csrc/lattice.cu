@@ -15,6 +15,7 @@
 #include "d3q19.cuh"
 #include "lattice_internal.h"
 #include "sweep_tma.cuh"
+#include "sweep_t2.cuh"
 
 using namespace bgk;
 
@@ -104,6 +105,80 @@ int one_step(bgk_lattice* L, cudaStream_t st, double* mom = nullptr, double* mom
     return BGK_OK;
 }
 
+int two_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st) {
+    switch (L->p.kind) {
+        case K_F64: return launch_sweep_t2<double, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+        case K_F32: return launch_sweep_t2<float, float>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+        case K_F32_F64: return launch_sweep_t2<float, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+    }
+    return set_error(BGK_ERR_UNSUPPORTED, "two-step sweep: 4- and 8-byte kinds");
+}
+
+// True when the lattice's steps run four at a time as two launches of two
+// steps each (sweep_t2.cuh): where its 37 arrays outgrow the 126 MB L2.  Below
+// that the one-step sweep runs from L2 and the rims cost more than they save
+// (FP32 64^3, 62 MB: 41 GLUPS against 34; FP64 64^3, 124 MB: 26 against 25).
+// Where the line lies depends on the case, whose face and obstacle blocks
+// take longer: periodic 120 MB (FP32 80^3, 127 MB, 35.2 -> 37.4), walls 150 MB
+// (FP32 driven 80^3 34.6 against 30.1; 96^3, 182 MB, 36.6 -> 41.5), inflow 300 MB
+// (FP32 with a sphere 199x83x61, 203 MB, 31.7 against 28.8; 128^3, 400 MB, 34.9
+// -> 36.4).
+bool steps_in_fours(const bgk_lattice* L) {
+    const bool has_obs = L->p.obs && L->p.imin <= L->p.imax;
+    if (!L->rest || (has_obs && !L->links) || L->p.zhalo || (L->tma_ok && g_tma_kernels)) return false;
+    const size_t mb = L->p.bcase == BC_PERIODIC ? 120 : (L->p.bcase == BC_INFLOW ? 300 : 150);
+    return L->bytes >= (mb << 20);
+}
+
+// The table of solid links the two-step sweep reads (t2_links_kernel), made
+// for the lattice's current obstacle; without it (no memory left) the lattice
+// takes single steps.
+void make_links(bgk_lattice* L) {
+    if (!L->rest) return;
+    const bgk_sweep_params& p = L->p;
+    const long long nodes = (long long)(p.imax - p.imin + 3) * (p.jmax - p.jmin + 3) * (p.kmax - p.kmin + 3);
+    void* buf = nullptr;
+    if (dev_alloc(&buf, (size_t)nodes * sizeof(uint32_t), false, "solid links") != BGK_OK) return;
+    SweepArgs<float, float> A{};
+    A.obs = p.obs; A.obs_nx = p.obs_nx; A.obs_nxy = (long long)p.obs_nx * p.obs_ny;
+    A.imin = p.imin; A.imax = p.imax; A.jmin = p.jmin; A.jmax = p.jmax; A.kmin = p.kmin; A.kmax = p.kmax;
+    cudaStream_t s = setup_stream();
+    t2_links_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(A, static_cast<uint32_t*>(buf));
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) { dev_free(buf); return; }
+    L->links = static_cast<uint32_t*>(buf);
+}
+
+void drop_links(bgk_lattice* L) {
+    dev_free(L->links);
+    L->links = nullptr;
+}
+
+// Four steps as two launches a -> b -> a.  The arrays end as four single
+// steps leave them: the same arrays hold the state, and neither the halo nor
+// the solid nodes of either set are written (an inflow lattice's outflow
+// plane is, by both).  The rest population, which single steps update in
+// place, passes through L->rest.
+int four_steps(bgk_lattice* L, cudaStream_t st) {
+    void* b[19];
+    std::memcpy(b, L->b, sizeof b);
+    b[18] = L->rest;
+    if (int e = two_steps(L, L->a, b, L->outflow_fresh, st)) return e;
+    if (int e = two_steps(L, b, L->a, true, st)) return e;
+    L->outflow_fresh = L->p.bcase == BC_INFLOW;
+    L->steps += 4;
+    return BGK_OK;
+}
+
+// nsteps steps without the graph.
+int plain_steps(bgk_lattice* L, int nsteps, cudaStream_t st) {
+    if (steps_in_fours(L))
+        for (; nsteps >= 4; nsteps -= 4)
+            if (int e = four_steps(L, st)) return e;
+    for (; nsteps > 0; --nsteps)
+        if (int e = one_step(L, st)) return e;
+    return BGK_OK;
+}
+
 // Capture kGraphSteps steps (starting from an even step count, so the
 // pointer arrangement / slot layout after the graph equals the one before).
 int build_graph(bgk_lattice* L) {
@@ -121,8 +196,7 @@ int build_graph(bgk_lattice* L) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(L->cap_stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) { L->outflow_fresh = fresh0; return set_error(BGK_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e)); }
-    int rc = BGK_OK;
-    for (int s = 0; s < kGraphSteps && rc == BGK_OK; ++s) rc = one_step(L, L->cap_stream);
+    const int rc = plain_steps(L, kGraphSteps, L->cap_stream);
     e = cudaStreamEndCapture(L->cap_stream, &g);
     L->graph_fresh = L->outflow_fresh;
     L->outflow_fresh = fresh0;
@@ -311,6 +385,15 @@ int bgk_lattice_create(const bgk_lattice_desc* d, bgk_lattice** out) {
         return rc;
     }
     make_tensor_map(L);
+    // the rest population's second buffer for the two-step sweep (32-bit byte
+    // offsets); without it (no memory left) the lattice takes single steps
+    if (d->pattern == BGK_PATTERN_AB && L->es >= 4 && (L->nx * L->ny * L->nz + 64) * L->es < (1LL << 32)) {
+        void* buf = nullptr;
+        if (dev_alloc(&buf, (size_t)L->plane * L->es, false, "rest population") == BGK_OK) {
+            L->rest_base = static_cast<char*>(buf);
+            L->rest = L->rest_base + (size_t)(L->shift + L->origin) * L->es;
+        }
+    }
     *out = L;
     return BGK_OK;
 }
@@ -320,7 +403,7 @@ int bgk_lattice_status(const bgk_lattice* L) {
     int flag = 0;
     const cudaError_t e = cudaMemcpy(&flag, L->err, sizeof(int), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "status: %s", cudaGetErrorString(e));
-    if (flag) return set_error(BGK_ERR_CUDA, "a TMA sweep gave up waiting for its copies; the state is undefined");
+    if (flag) return set_error(BGK_ERR_CUDA, "a sweep gave up waiting inside the GPU; the state is undefined");
     return BGK_OK;
 }
 
@@ -367,6 +450,8 @@ int bgk_lattice_destroy_async(bgk_lattice* L, void* stream) {
     drop_graph(L);
     if (L->cap_stream) cudaStreamDestroy(L->cap_stream);
     dev_free_async(L->base, st);
+    dev_free_async(L->rest_base, st);
+    dev_free_async(L->links, st);
     dev_free_async(L->obs_dev, st);
     dev_free_async(L->ws, st);
     dev_free_async(L->mom, st);
@@ -380,6 +465,8 @@ int bgk_lattice_destroy(bgk_lattice* L) {
     drop_graph(L);
     if (L->cap_stream) cudaStreamDestroy(L->cap_stream);
     dev_free(L->base);
+    dev_free(L->rest_base);
+    dev_free(L->links);
     dev_free(L->obs_dev);
     dev_free(L->ws);
     dev_free(L->mom);
@@ -391,6 +478,7 @@ int bgk_lattice_destroy(bgk_lattice* L) {
 int bgk_lattice_set_sphere(bgk_lattice* L, double cx, double cy, double cz, double r2) {
     if (!L) return set_error(BGK_ERR_ARG, "null lattice");
     drop_graph(L);
+    drop_links(L);
     dev_free(L->obs_dev);
     L->obs_dev = nullptr;
     L->p.obs = nullptr;
@@ -420,12 +508,14 @@ int bgk_lattice_set_sphere(bgk_lattice* L, double cx, double cy, double cz, doub
     if (int err = validate(&q)) { dev_free(obs); return err; }
     L->obs_dev = obs;
     L->p = q;
+    make_links(L);
     return BGK_OK;
 }
 
 int bgk_lattice_set_obstacle(bgk_lattice* L, const int32_t* obs) {
     if (!L) return set_error(BGK_ERR_ARG, "null lattice");
     drop_graph(L);
+    drop_links(L);
     dev_free(L->obs_dev);
     L->obs_dev = nullptr;
     L->p.obs = nullptr;
@@ -458,6 +548,7 @@ int bgk_lattice_set_obstacle(bgk_lattice* L, const int32_t* obs) {
     }
     q.obs = L->obs_dev;
     L->p = q;
+    make_links(L);
     return BGK_OK;
 }
 
@@ -553,9 +644,7 @@ int bgk_lattice_step(bgk_lattice* L, int nsteps, void* stream) {
             L->outflow_fresh = L->graph_fresh;
         }
     }
-    while (left-- > 0)
-        if (int e = one_step(L, st)) return e;
-    return BGK_OK;
+    return plain_steps(L, left, st);
 }
 
 int bgk_lattice_step_moments(bgk_lattice* L, int nsteps, int every, double* out_dev, void* stream) {

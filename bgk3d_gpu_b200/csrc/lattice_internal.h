@@ -18,6 +18,9 @@ struct bgk_lattice {
     std::vector<void*> planes;   // plane pointers at element (0,0,0)
     void* a[19];                 // AB: current populations; AA: slot arrays
     void* b[19];                 // AB: next populations (b[18] = a[18])
+    char* rest_base = nullptr;   // AB: a second array of population 19 (two-step sweep), or null
+    void* rest = nullptr;        // its element (0,0,0)
+    uint32_t* links = nullptr;   // with an obstacle: its table of solid links (two-step sweep), or null
     int32_t* obs_dev = nullptr;
     long long steps = 0;
     double* ws = nullptr;
@@ -29,7 +32,7 @@ struct bgk_lattice {
     size_t mom_bytes = 0;
     alignas(64) CUtensorMap tmap; // the allocation as x, y, z, plane (sweep_tma.cuh)
     bool tma_ok = false;         // tmap is valid (AB pattern, driver support)
-    int* err = nullptr;          // device flag set by a TMA kernel wait that gave up
+    int* err = nullptr;          // device flag set by a wait of a TMA or two-step sweep that gave up
     // inflow, AB: the current a arrays' outflow plane holds the equilibria of
     // the current state (the last step wrote it), so the next step needs no
     // pre-pass; graph_fresh: the same after a replay of the step graph

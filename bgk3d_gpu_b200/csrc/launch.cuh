@@ -2,12 +2,14 @@
 // kind by the inst_*.cu translation units; declared in kernels.h.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cuda_runtime.h>
 #include "bgk3d_b200.h"
 #include "bgk_internal.h"
 #include "host_args.cuh"
 #include "sweep_ab.cuh"
 #include "sweep_aa.cuh"
+#include "sweep_t2.cuh"
 #include "sweep_tma.cuh"
 #include "reduce.cuh"
 #include "batch.cuh"
@@ -227,6 +229,75 @@ int launch_sweep(const bgk_sweep_params* p, void* const* a, void* const* b, doub
         case BC_INFLOW: by_variant<AbLaunch, S, C, BC_INFLOW>(nelem, cm, obs, A, nb, st); break;
     }
     return check_launch("sweep_ab_kernel");
+}
+
+// Two steps in one launch (sweep_t2.cuh).  a and b: 19 arrays each (b[18] a
+// buffer of its own: the rest population is not updated in place here).
+template <class S, class C, int BC, int CM, bool OBS>
+int launch_t2_variant(const SweepArgs<S, C>& A, const uint32_t* links, int* err, cudaStream_t st) {
+    typedef T2Lay<S, C, BC, OBS> R;
+    auto kern = sweep_t2_kernel<S, C, BC, CM, OBS>;
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    static std::atomic<unsigned long long> ready{0};   // devices on which the kernel's shared-memory limit is raised
+    if (!(ready.load(std::memory_order_acquire) >> (dev & 63) & 1)) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, R::BYTES);
+        if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "two-step sweep: %s", cudaGetErrorString(e));
+        ready.fetch_or(1ULL << (dev & 63), std::memory_order_release);
+    }
+    T2Args<S, C> Q;
+    Q.s = A;
+    Q.links = links;
+    Q.err = err;
+    for (int d = 0; d < 19; ++d) Q.src[d] = A.a[d] - (cx_of(d) + cy_of(d) * A.nx + cz_of(d) * A.nxy);
+    Q.g = t2_tiles(A.l, A.m, A.n, R::TX, R::H, nsm * T2Cfg<C>::BLOCKS, t2_uneven<C, BC>(OBS));
+    const long long units = (long long)Q.g.ntx * Q.g.nty * ((A.n + Q.g.zc - 1) / Q.g.zc);
+    kern<<<(unsigned)units, R::THREADS, R::BYTES, st>>>(Q);
+    return check_launch("sweep_t2_kernel");
+}
+
+template <class S, class C, int BC, bool OBS>
+int launch_t2_cm(const SweepArgs<S, C>& A, int cm, const uint32_t* links, int* err, cudaStream_t st) {
+    switch (cm) {
+        case CM_STRICT: return launch_t2_variant<S, C, BC, CM_STRICT, OBS>(A, links, err, st);
+        case CM_STRICT_GENERIC: return launch_t2_variant<S, C, BC, CM_STRICT_GENERIC, OBS>(A, links, err, st);
+        case CM_FAST:
+            if constexpr (sizeof(C) == 4) return launch_t2_variant<S, C, BC, CM_FAST, OBS>(A, links, err, st);
+            break;
+        default:
+            if constexpr (sizeof(C) == 4) return launch_t2_variant<S, C, BC, CM_FAST_GENERIC, OBS>(A, links, err, st);
+            break;
+    }
+    return set_error(BGK_ERR_ARG, "collision mode %d", cm);
+}
+
+template <class S, class C, int BC>
+int launch_t2_bc(const SweepArgs<S, C>& A, const uint32_t* links, int* err, cudaStream_t st) {
+    const int cm = coll_mode(A);
+    if (A.obs) return launch_t2_cm<S, C, BC, true>(A, cm, links, err, st);
+    return launch_t2_cm<S, C, BC, false>(A, cm, nullptr, err, st);
+}
+
+// outflow_fresh (inflow case): a's outflow plane holds the equilibria of a's
+// state already; the launch always writes the next state's into b.
+template <class S, class C>
+int launch_sweep_t2(const bgk_sweep_params* p, void* const* a, void* const* b, const uint32_t* links, int* err,
+                    bool outflow_fresh, cudaStream_t st) {
+    SweepArgs<S, C> A = sweep_args<S, C>(p, a, b);
+    A.b[18] = (S*)b[18];
+    if (p->bcase == BC_INFLOW && !outflow_fresh) {
+        dim3 blk(128), grd((p->m + 127) / 128, p->n);
+        outflow_halo_kernel<S, C><<<grd, blk, 0, st>>>(A);
+        if (int e = check_launch("outflow_halo_kernel")) return e;
+    }
+    switch (p->bcase) {
+        case BC_DRIVEN: return launch_t2_bc<S, C, BC_DRIVEN>(A, links, err, st);
+        case BC_PERIODIC: return launch_t2_bc<S, C, BC_PERIODIC>(A, links, err, st);
+        case BC_CHANNEL: return launch_t2_bc<S, C, BC_CHANNEL>(A, links, err, st);
+        case BC_INFLOW: return launch_t2_bc<S, C, BC_INFLOW>(A, links, err, st);
+    }
+    return set_error(BGK_ERR_ARG, "the two-step sweep needs a boundary case");
 }
 
 // TMA-staged sweep (sweep_tma.cuh) for library-owned AB lattices without
@@ -620,6 +691,11 @@ int launch_init(void* const* f, long long nx, long long ny, int l, int m, int n,
                                     cudaStream_t, int*, double*, unsigned*);                       \
     template int launch_sweep_tma<S, C>(const bgk_sweep_params*, void* const*, void* const*,        \
                                         const void*, const int*, int*, cudaStream_t);              \
+    }
+#define BGK_INSTANTIATE_T2(S, C)                                                                   \
+    namespace bgk {                                                                                \
+    template int launch_sweep_t2<S, C>(const bgk_sweep_params*, void* const*, void* const*,        \
+                                       const uint32_t*, int*, bool, cudaStream_t);                 \
     }
 #define BGK_INSTANTIATE_AA(S, C)                                                                   \
     namespace bgk {                                                                                \

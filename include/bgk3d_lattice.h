@@ -44,7 +44,11 @@ typedef struct bgk_lattice_desc {
 /* Defaults: AB pattern, no force, lid 0, inflow 0, scale 1, fast 0. */
 void bgk_lattice_desc_init(bgk_lattice_desc* d, int kind, int bcase, int l, int m, int n, double omega);
 
-/* Device bytes a lattice with this description occupies (admission control). */
+/* Device bytes a lattice with this description needs (admission control).  An
+   AB lattice of a 4- or 8-byte kind takes one more population array (1/37)
+   where the device has room for it, and with an obstacle 4 bytes per node of
+   the obstacle's box: what its two-step launches work with.  Without them it
+   takes single steps. */
 size_t bgk_lattice_device_bytes(const bgk_lattice_desc* d);
 
 /* Allocate the lattice on the current device.  Lattices, batches and their
@@ -129,7 +133,10 @@ long long bgk_io_set_subrecord_limit(long long bytes);
 
 /* Advance nsteps time steps (boundaries + stream + collide), stream-ordered.
    Runs of 32 or more steps replay a captured 16-step CUDA graph (captured on
-   the first such run unless bgk_lattice_prepare captured it before). */
+   the first such run unless bgk_lattice_prepare captured it before).  AB
+   lattices of the 4- and 8-byte kinds whose arrays outgrow the L2 cache take
+   four steps at a time as two launches of two steps each; the result is bit
+   for bit that of single steps. */
 int bgk_lattice_step(bgk_lattice* lat, int nsteps, void* stream);
 
 /* Capture the 16-step CUDA graph of bgk_lattice_step now, without running
@@ -180,7 +187,8 @@ int bgk_lattice_slice(const bgk_lattice* lat, int plane, int index, float* out_d
    returns the previous setting (not thread-safe against concurrent launches).
    bgk_lattice_status: BGK_ERR_CUDA when a TMA sweep gave up waiting for its
    copies (about one second; the kernel then returns and the state is
-   undefined), else BGK_OK; synchronous.  No counterpart in the reference. */
+   undefined) or a two-step launch for its block's warps, else BGK_OK;
+   synchronous.  No counterpart in the reference. */
 int bgk_lattice_uses_tma(const bgk_lattice* lat);
 int bgk_set_tma_kernels(int enable);
 int bgk_lattice_status(const bgk_lattice* lat);

@@ -51,6 +51,13 @@ struct bgk_batch {
     // graph branches of the grouped form: work items (solo member: its index;
     // group g: -1 - g) spread over up to kBranches branches
     std::vector<std::vector<int>> branches;
+    // Members whose steps run four at a time (bgk_lat::four_steps), and the
+    // groups of the others: what the grouped form takes while four or more
+    // steps are left.  The groups above hold every member and take the
+    // remainder, one step at a time.
+    std::vector<char> in_fours;
+    std::vector<Group> others;
+    std::vector<std::vector<int>> four_branches;   // like branches, over in_fours members, solo members and others
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> ev;          // fork + one join per branch
 };
@@ -170,23 +177,45 @@ int build_groups(bgk_batch* B) {
         g->members.push_back((int)i);
     }
     // work items, largest first, each onto the branch with the fewest nodes
-    std::vector<std::pair<long long, int>> items;
-    for (int i : B->solo) items.push_back({member_nodes(B, i), i});
-    for (size_t g = 0; g < B->groups.size(); ++g) {
-        long long nodes = 0;
-        for (int i : B->groups[g].members) nodes += member_nodes(B, i);
-        items.push_back({nodes, -1 - (int)g});
-    }
-    std::stable_sort(items.begin(), items.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-    const size_t nb = std::min<size_t>(kBranches, items.size());
-    B->branches.assign(nb, {});
-    std::vector<long long> load(nb, 0);
-    for (const auto& it : items) {
-        const size_t t = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
-        B->branches[t].push_back(it.second);
-        load[t] += it.first;
-    }
+    auto spread = [&](const std::vector<int>& alone, const std::vector<bgk_batch::Group>& groups,
+                      std::vector<std::vector<int>>& branches) {
+        std::vector<std::pair<long long, int>> items;
+        for (int i : alone) items.push_back({member_nodes(B, i), i});
+        for (size_t g = 0; g < groups.size(); ++g) {
+            long long nodes = 0;
+            for (int i : groups[g].members) nodes += member_nodes(B, i);
+            items.push_back({nodes, -1 - (int)g});
+        }
+        std::stable_sort(items.begin(), items.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+        const size_t nb = std::min<size_t>(kBranches, items.size());
+        branches.assign(nb, {});
+        std::vector<long long> load(nb, 0);
+        for (const auto& it : items) {
+            const size_t t = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
+            branches[t].push_back(it.second);
+            load[t] += it.first;
+        }
+    };
+    spread(B->solo, B->groups, B->branches);
+    // the same for rounds of four steps: members that take them at a time
+    // leave their groups
+    B->in_fours.assign(B->lats.size(), 0);
+    B->others.clear();
+    B->four_branches.clear();
     if (B->chunk <= 0) return BGK_OK;
+    std::vector<int> alone;
+    for (size_t i = 0; i < B->lats.size(); ++i) {
+        B->in_fours[i] = bgk_lat::steps_in_fours(B->lats[i]) ? 1 : 0;
+        if (B->in_fours[i] || std::find(B->solo.begin(), B->solo.end(), (int)i) != B->solo.end()) alone.push_back((int)i);
+    }
+    for (const bgk_batch::Group& g : B->groups) {
+        bgk_batch::Group o = g;
+        o.members.clear();
+        for (int i : g.members)
+            if (!B->in_fours[i]) o.members.push_back(i);
+        if (!o.members.empty()) B->others.push_back(o);
+    }
+    if (std::count(B->in_fours.begin(), B->in_fours.end(), 1)) spread(alone, B->others, B->four_branches);
     // launches of earlier steps may still read the current table (they run
     // asynchronously on the caller's stream): wait for them before the table
     // is rewritten in place
@@ -195,14 +224,15 @@ int build_groups(bgk_batch* B) {
         if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "chunk table: %s", cudaGetErrorString(e));
     }
     std::vector<uint2> table;
-    for (bgk_batch::Group& g : B->groups) {
-        g.first = table.size();
-        for (int i : g.members) {
-            const long long w = member_warps(B->lats[i]);
-            for (long long c = 0; c < w; c += B->chunk) table.push_back(make_uint2((unsigned)i, (unsigned)c));
+    for (std::vector<bgk_batch::Group>* groups : {&B->groups, &B->others})
+        for (bgk_batch::Group& g : *groups) {
+            g.first = table.size();
+            for (int i : g.members) {
+                const long long w = member_warps(B->lats[i]);
+                for (long long c = 0; c < w; c += B->chunk) table.push_back(make_uint2((unsigned)i, (unsigned)c));
+            }
+            g.nchunks = (uint32_t)(table.size() - g.first);
         }
-        g.nchunks = (uint32_t)(table.size() - g.first);
-    }
     if (table.size() > B->chunk_cap) {
         dev_free(B->chunks);
         B->chunks = nullptr;
@@ -248,11 +278,31 @@ int item_step(bgk_batch* B, int item, int par, cudaStream_t st) {
     return group_step(B, B->groups[(size_t)(-1 - item)], par, st);
 }
 
+// Four steps of a work item of four_branches from batch parity par (member
+// idx >= 0, or group -1 - idx of the others).
+int item_four(bgk_batch* B, int item, int par, cudaStream_t st) {
+    if (item >= 0 && B->in_fours[(size_t)item]) {
+        void* a[19];
+        void* b[19];
+        member_arrays(B, (size_t)item, par, a);
+        member_arrays(B, (size_t)item, par ^ 1, b);
+        return bgk_lat::four_steps(B->lats[(size_t)item], a, b, false, st);
+    }
+    for (int s = 0; s < 4; ++s) {
+        const int e = item >= 0 ? member_step(B, item, par ^ (s & 1), st)
+                                : group_step(B, B->others[(size_t)(-1 - item)], par ^ (s & 1), st);
+        if (e) return e;
+    }
+    return BGK_OK;
+}
+
 // Graph of kBatchGraphSteps steps of the grouped form: the work items are
 // independent lattices, so each branch runs its items' chains of steps
 // (fork / join), and one item's last wave overlaps the others' work.
 int capture_branches(bgk_batch* B) {
-    const size_t G = B->branches.size();
+    const bool fours = !B->four_branches.empty();
+    const std::vector<std::vector<int>>& branches = fours ? B->four_branches : B->branches;
+    const size_t G = branches.size();
     while (B->side.size() < G) {
         cudaStream_t s = nullptr;
         cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
@@ -268,9 +318,9 @@ int capture_branches(bgk_batch* B) {
     if (cudaEventRecord(B->ev[0], B->cap) != cudaSuccess) return set_error(BGK_ERR_CUDA, "fork record");
     for (size_t g = 0; g < G; ++g) {
         if (cudaStreamWaitEvent(B->side[g], B->ev[0], 0) != cudaSuccess) return set_error(BGK_ERR_CUDA, "fork wait");
-        for (int s = 0; s < kBatchGraphSteps; ++s)
-            for (int item : B->branches[g])
-                if (int e = item_step(B, item, s & 1, B->side[g])) return e;
+        for (int s = 0; s < kBatchGraphSteps; s += fours ? 4 : 1)
+            for (int item : branches[g])
+                if (int e = fours ? item_four(B, item, 0, B->side[g]) : item_step(B, item, s & 1, B->side[g])) return e;
         if (cudaEventRecord(B->ev[g + 1], B->side[g]) != cudaSuccess) return set_error(BGK_ERR_CUDA, "join record");
         if (cudaStreamWaitEvent(B->cap, B->ev[g + 1], 0) != cudaSuccess) return set_error(BGK_ERR_CUDA, "join wait");
     }
@@ -293,6 +343,21 @@ int batch_one(bgk_batch* B, cudaStream_t st) {
         if (int e = batch_launch(B, par, st)) return e;
     }
     ++B->steps;
+    return BGK_OK;
+}
+
+// nsteps batch steps without the graph: rounds of four where members take
+// them, then single steps.
+int batch_plain(bgk_batch* B, int nsteps, cudaStream_t st) {
+    if (!B->four_branches.empty())
+        for (; nsteps >= 4; nsteps -= 4) {
+            for (const std::vector<int>& br : B->four_branches)
+                for (int item : br)
+                    if (int e = item_four(B, item, (int)(B->steps & 1), st)) return e;
+            B->steps += 4;
+        }
+    for (; nsteps > 0; --nsteps)
+        if (int e = batch_one(B, st)) return e;
     return BGK_OK;
 }
 
@@ -324,9 +389,8 @@ int build_graph(bgk_batch* B) {
     cudaError_t e = cudaStreamBeginCapture(B->cap, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     int rc = BGK_OK;
-    if (B->chunk > 0 && B->branches.size() > 1) rc = capture_branches(B);
-    else
-        for (int s = 0; s < kBatchGraphSteps && rc == BGK_OK; ++s) rc = batch_one(B, B->cap);
+    if (B->chunk > 0 && std::max(B->branches.size(), B->four_branches.size()) > 1) rc = capture_branches(B);
+    else rc = batch_plain(B, kBatchGraphSteps, B->cap);
     e = cudaStreamEndCapture(B->cap, &g);
     B->steps = saved;
     if (rc != BGK_OK) { if (g) cudaGraphDestroy(g); return rc; }
@@ -355,9 +419,7 @@ int run_steps(bgk_batch* B, int nsteps, cudaStream_t st) {
             left -= B->graph_steps;
         }
     }
-    while (left-- > 0)
-        if (int e = batch_one(B, st)) return e;
-    return BGK_OK;
+    return batch_plain(B, left, st);
 }
 
 }  // namespace

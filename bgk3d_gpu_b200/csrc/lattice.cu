@@ -105,29 +105,17 @@ int one_step(bgk_lattice* L, cudaStream_t st, double* mom = nullptr, double* mom
     return BGK_OK;
 }
 
-int two_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st) {
-    switch (L->p.kind) {
-        case K_F64: return launch_sweep_t2<double, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
-        case K_F32: return launch_sweep_t2<float, float>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
-        case K_F32_F64: return launch_sweep_t2<float, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
-    }
-    return set_error(BGK_ERR_UNSUPPORTED, "two-step sweep: 4- and 8-byte kinds");
-}
-
-// True when the lattice's steps run four at a time as two launches of two
-// steps each (sweep_t2.cuh): where its 37 arrays outgrow the 126 MB L2.  Below
-// that the one-step sweep runs from L2 and the rims cost more than they save
+// Bytes of a lattice's arrays from which its steps run four at a time, as two
+// launches of two steps each (sweep_t2.cuh): where they outgrow the 126 MB L2.
+// Below that the one-step sweep runs from L2 and the rims cost more than they save
 // (FP32 64^3, 62 MB: 41 GLUPS against 34; FP64 64^3, 124 MB: 26 against 25).
 // Where the line lies depends on the case, whose face and obstacle blocks
 // take longer: periodic 120 MB (FP32 80^3, 127 MB, 35.2 -> 37.4), walls 150 MB
 // (FP32 driven 80^3 34.6 against 30.1; 96^3, 182 MB, 36.6 -> 41.5), inflow 300 MB
 // (FP32 with a sphere 199x83x61, 203 MB, 31.7 against 28.8; 128^3, 400 MB, 34.9
 // -> 36.4).
-bool steps_in_fours(const bgk_lattice* L) {
-    const bool has_obs = L->p.obs && L->p.imin <= L->p.imax;
-    if (!L->rest || (has_obs && !L->links) || L->p.zhalo || (L->tma_ok && g_tma_kernels)) return false;
-    const size_t mb = L->p.bcase == BC_PERIODIC ? 120 : (L->p.bcase == BC_INFLOW ? 300 : 150);
-    return L->bytes >= (mb << 20);
+size_t two_step_line(int bcase) {
+    return (size_t)(bcase == BC_PERIODIC ? 120 : (bcase == BC_INFLOW ? 300 : 150)) << 20;
 }
 
 // The table of solid links the two-step sweep reads (t2_links_kernel), made
@@ -153,27 +141,14 @@ void drop_links(bgk_lattice* L) {
     L->links = nullptr;
 }
 
-// Four steps as two launches a -> b -> a.  The arrays end as four single
-// steps leave them: the same arrays hold the state, and neither the halo nor
-// the solid nodes of either set are written (an inflow lattice's outflow
-// plane is, by both).  The rest population, which single steps update in
-// place, passes through L->rest.
-int four_steps(bgk_lattice* L, cudaStream_t st) {
-    void* b[19];
-    std::memcpy(b, L->b, sizeof b);
-    b[18] = L->rest;
-    if (int e = two_steps(L, L->a, b, L->outflow_fresh, st)) return e;
-    if (int e = two_steps(L, b, L->a, true, st)) return e;
-    L->outflow_fresh = L->p.bcase == BC_INFLOW;
-    L->steps += 4;
-    return BGK_OK;
-}
-
 // nsteps steps without the graph.
 int plain_steps(bgk_lattice* L, int nsteps, cudaStream_t st) {
-    if (steps_in_fours(L))
-        for (; nsteps >= 4; nsteps -= 4)
-            if (int e = four_steps(L, st)) return e;
+    if (bgk_lat::steps_in_fours(L) && !(L->tma_ok && g_tma_kernels))
+        for (; nsteps >= 4; nsteps -= 4) {
+            if (int e = bgk_lat::four_steps(L, L->a, L->b, L->outflow_fresh, st)) return e;
+            L->outflow_fresh = L->p.bcase == BC_INFLOW;
+            L->steps += 4;
+        }
     for (; nsteps > 0; --nsteps)
         if (int e = one_step(L, st)) return e;
     return BGK_OK;
@@ -304,6 +279,27 @@ int tma_step(bgk_lattice* L, cudaStream_t st) {
 }  // namespace
 
 namespace bgk_lat {
+static int two_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st) {
+    switch (L->p.kind) {
+        case K_F64: return launch_sweep_t2<double, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+        case K_F32: return launch_sweep_t2<float, float>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+        case K_F32_F64: return launch_sweep_t2<float, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+    }
+    return set_error(BGK_ERR_UNSUPPORTED, "two-step sweep: 4- and 8-byte kinds");
+}
+
+bool steps_in_fours(const bgk_lattice* L) {
+    const bool has_obs = L->p.obs && L->p.imin <= L->p.imax;
+    return L->rest && (!has_obs || L->links) && !L->p.zhalo;
+}
+
+int four_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st) {
+    void* t[19];
+    for (int d = 0; d < 19; ++d) t[d] = d < 18 ? b[d] : L->rest;
+    if (int e = two_steps(L, a, t, outflow_fresh, st)) return e;
+    return two_steps(L, t, a, true, st);
+}
+
 void observable(const bgk_lattice* L, void** out) {
     if (L->desc.pattern == BGK_PATTERN_AA)
         for (int d = 0; d < 19; ++d) out[d] = L->a[opp_of(d)];
@@ -365,7 +361,15 @@ int bgk_lattice_create(const bgk_lattice_desc* d, bgk_lattice** out) {
     L->p.fast = d->fast;
     if (int e = validate(&L->p)) { delete L; return e; }
     L->bytes = bgk_lattice_device_bytes(d);
-    if (int rc = dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes, true, "lattice")) {
+    // a lattice whose steps run four at a time has one array more, the rest
+    // population's second one (two-step sweep, 32-bit byte offsets), in the
+    // same block of memory; without room for it, it takes single steps
+    const size_t array = (size_t)L->plane * L->es;
+    const bool fours = d->pattern == BGK_PATTERN_AB && L->es >= 4 && L->bytes >= two_step_line(d->bcase) && array < (1ULL << 32);
+    int rc = fours ? dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes + array, true, "lattice") : BGK_ERR_NOMEM;
+    if (rc == BGK_OK) L->rest = L->base + L->bytes + (size_t)(L->shift + L->origin) * L->es;
+    else rc = dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes, true, "lattice");
+    if (rc) {
         delete L;
         return rc;
     }
@@ -379,21 +383,12 @@ int bgk_lattice_create(const bgk_lattice_desc* d, bgk_lattice** out) {
     } else {
         for (int q = 0; q < 19; ++q) L->b[q] = L->a[q];
     }
-    if (int rc = dev_alloc(reinterpret_cast<void**>(&L->err), sizeof(int), true, "status flag")) {
+    if ((rc = dev_alloc(reinterpret_cast<void**>(&L->err), sizeof(int), true, "status flag"))) {
         dev_free(L->base);
         delete L;
         return rc;
     }
     make_tensor_map(L);
-    // the rest population's second buffer for the two-step sweep (32-bit byte
-    // offsets); without it (no memory left) the lattice takes single steps
-    if (d->pattern == BGK_PATTERN_AB && L->es >= 4 && (L->nx * L->ny * L->nz + 64) * L->es < (1LL << 32)) {
-        void* buf = nullptr;
-        if (dev_alloc(&buf, (size_t)L->plane * L->es, false, "rest population") == BGK_OK) {
-            L->rest_base = static_cast<char*>(buf);
-            L->rest = L->rest_base + (size_t)(L->shift + L->origin) * L->es;
-        }
-    }
     *out = L;
     return BGK_OK;
 }
@@ -450,7 +445,6 @@ int bgk_lattice_destroy_async(bgk_lattice* L, void* stream) {
     drop_graph(L);
     if (L->cap_stream) cudaStreamDestroy(L->cap_stream);
     dev_free_async(L->base, st);
-    dev_free_async(L->rest_base, st);
     dev_free_async(L->links, st);
     dev_free_async(L->obs_dev, st);
     dev_free_async(L->ws, st);
@@ -465,7 +459,6 @@ int bgk_lattice_destroy(bgk_lattice* L) {
     drop_graph(L);
     if (L->cap_stream) cudaStreamDestroy(L->cap_stream);
     dev_free(L->base);
-    dev_free(L->rest_base);
     dev_free(L->links);
     dev_free(L->obs_dev);
     dev_free(L->ws);

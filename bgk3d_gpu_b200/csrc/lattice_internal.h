@@ -18,8 +18,7 @@ struct bgk_lattice {
     std::vector<void*> planes;   // plane pointers at element (0,0,0)
     void* a[19];                 // AB: current populations; AA: slot arrays
     void* b[19];                 // AB: next populations (b[18] = a[18])
-    char* rest_base = nullptr;   // AB: a second array of population 19 (two-step sweep), or null
-    void* rest = nullptr;        // its element (0,0,0)
+    void* rest = nullptr;        // AB, large: a second array of population 19 at element (0,0,0) (two-step sweep), or null
     uint32_t* links = nullptr;   // with an obstacle: its table of solid links (two-step sweep), or null
     int32_t* obs_dev = nullptr;
     long long steps = 0;
@@ -40,8 +39,19 @@ struct bgk_lattice {
     bool graph_fresh = false;
 };
 
-// Shared by the lattice's host-transfer paths (lattice.cu, lattice_io.cu).
+// Shared by the lattice's host-transfer paths (lattice.cu, lattice_io.cu) and
+// the batched stepper.
 namespace bgk_lat {
+// True when the lattice's steps run four at a time (AB, arrays that outgrow
+// L2, rest population's second array and obstacle table in place).
+bool steps_in_fours(const bgk_lattice* L);
+// Four steps as two two-step launches a -> b -> a.  The arrays end as four
+// single steps leave them: a holds the state, and neither the halo nor the
+// solid nodes of either set are written (an inflow lattice's outflow plane
+// is, by both).  The rest population, which single steps update in place,
+// passes through L->rest.  outflow_fresh: a's outflow plane needs no pre-pass
+// (it needs none afterwards either).
+int four_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st);
 // Device arrays holding populations 01..19 of the observable state.
 void observable(const bgk_lattice* L, void** out);
 // Reset the pointer arrangement to the base planes and return the arrays a

@@ -69,3 +69,34 @@ def test_two_steps_per_launch_with_solid_nodes(case, kind, fast):
 def test_graph_of_two_step_launches(case):
     """37 steps: a single step to an even count does not occur, two graph replays and a remainder of five."""
     assert_same(both(*SHAPES[case][0], 1, case, steps=37, fast=True), case)
+
+
+@pytest.mark.parametrize("steps", [5, 23])
+def test_batch_members_that_take_two_steps_per_launch(steps):
+    """A batch of members above and below the dispatch's line, stepped plainly
+    (5: a round of four and one) and through its graph (23: two replays, a
+    round and three), against every lattice stepped alone by single steps."""
+    from bgk3d_gpu_b200.lattice import Batch, Lattice
+    from test_gpu_lattice import lattice_kwargs
+    specs = [("periodic", (133, 97, 49)), ("channel", (20, 18, 16)), ("driven", (199, 83, 61)), ("channel", (101, 131, 67)),
+             ("inflow", (150, 131, 101)), ("periodic", (24, 20, 22))]
+    lats = {True: [], False: []}
+    for q, (case, (l, m, n)) in enumerate(specs):
+        st0 = random_state(l, m, n, 1, seed=q)
+        for alone in (True, False):
+            lat = Lattice(l, m, n, kind=1, bcase=BCASE[case], omega=OMEGA, **lattice_kwargs(case))
+            if case == "inflow":
+                lat.set_obstacle(scattered_solids(l, m, n, 9))
+            lat.upload(st0)
+            lats[alone].append(lat)
+    batch = Batch(lats[False])
+    batch.step(steps)
+    for lat in lats[True]:
+        for _ in range(steps):
+            lat.step(1)
+    for (case, shape), a, b in zip(specs, lats[True], lats[False]):
+        assert a.steps == b.steps
+        assert np.array_equal(a.download(), b.download()), f"{case} {shape}"
+    batch.close()
+    for lat in lats[True] + lats[False]:
+        lat.close()

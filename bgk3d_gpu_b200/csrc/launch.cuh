@@ -251,7 +251,8 @@ int launch_t2_variant(const SweepArgs<S, C>& A, const uint32_t* links, int* err,
     Q.links = links;
     Q.err = err;
     for (int d = 0; d < 19; ++d) Q.src[d] = A.a[d] - (cx_of(d) + cy_of(d) * A.nx + cz_of(d) * A.nxy);
-    Q.g = t2_tiles(A.l, A.m, A.n, R::TX, R::H, nsm * T2Cfg<C>::BLOCKS, t2_uneven<C, BC>(OBS));
+    Q.g = t2_tiles(A.l, A.m, A.n, R::TX, R::H, nsm * T2Cfg<C>::BLOCKS, t2_uneven<BC>(OBS),
+                     sizeof(C) == 4 ? 0.5 : 0.85);
     const long long units = (long long)Q.g.ntx * Q.g.nty * ((A.n + Q.g.zc - 1) / Q.g.zc);
     kern<<<(unsigned)units, R::THREADS, R::BYTES, st>>>(Q);
     return check_launch("sweep_t2_kernel");

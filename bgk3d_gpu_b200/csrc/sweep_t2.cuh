@@ -93,8 +93,8 @@ template <class S, class C, int BC, bool OBS> struct T2Lay {
 // How much longer than the others a block at a face or an obstacle takes (a
 // part of a block's time), which the last blocks to run show: with it FP32
 // driven 128^3 runs in two chunks instead of one, 102.9 -> 96.1 us per launch.
-template <class C, int BC> constexpr double t2_uneven(bool obs) {
-    return (BC == BC_PERIODIC ? 0.0 : (sizeof(C) == 4 ? 0.25 : 0.08)) + (obs ? 0.5 : 0.0);
+template <int BC> constexpr double t2_uneven(bool obs) {
+    return (BC == BC_PERIODIC ? 0.0 : 0.08) + (obs ? 0.5 : 0.0);
 }
 
 // The tiles of an l x m x n lattice (rows: of the largest tile and its rim;
@@ -102,11 +102,12 @@ template <class C, int BC> constexpr double t2_uneven(bool obs) {
 // fastest at every size tried (less of a plane is rim), so only the chunk
 // length is chosen: short chunks repeat more planes (two per chunk) and fill
 // more often, long ones leave slots idle at the end.  The cost counts nodes,
-// 250 per plane and 1000 per block for what does not depend on them, and runs
-// of blocks with half of the idle share of the last one.  Against all chunk
+// 250 per plane and 500 per block for what does not depend on them, and runs
+// of blocks with a part `idle` of the idle share of the last one (FP32 0.5,
+// whose blocks end more unevenly, FP64 0.85).  Against all chunk
 // lengths at nine sizes from 80^3 to 256^3 (FP32 and FP64, periodic and
-// driven): within 1.5 % of the fastest at 29 of 36, 6 % off at most.
-inline T2Tiles t2_tiles(int l, int m, int n, int txmax, int rows, int slots, double uneven) {
+// driven): 0.7 % (FP32) and 0.1 % (FP64) off the fastest on average, 3.6 % at most.
+inline T2Tiles t2_tiles(int l, int m, int n, int txmax, int rows, int slots, double uneven, double idle) {
     T2Tiles g;
     g.ntx = (l + txmax - 1) / txmax;
     g.tx = (l + g.ntx - 1) / g.ntx;
@@ -120,7 +121,7 @@ inline T2Tiles t2_tiles(int l, int m, int n, int txmax, int rows, int slots, dou
     for (long long nz = 1; nz <= n && (nz == 1 || (nz - 1) * tiles < 10LL * slots); ++nz) {
         const int zc = (int)((n + nz - 1) / nz);
         const double w = (double)(tiles * ((n + zc - 1) / zc)) / slots, up = std::ceil(w);
-        const double c = (w <= 1.0 ? 1.0 + uneven : w + 0.5 * (up - w) + uneven) * ((zc + 2) * n1 + zc * n2 + 1000.0);
+        const double c = (w <= 1.0 ? 1.0 + uneven : w + idle * (up - w) + uneven) * ((zc + 2) * n1 + zc * n2 + 500.0);
         if (g.zc == 0 || c < cost) { cost = c; g.zc = zc; }
     }
     return g;

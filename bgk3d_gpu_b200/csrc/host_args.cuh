@@ -132,6 +132,40 @@ void segment_geometry(SweepArgs<S, C>& A, const void* a0, bool allow_flat = fals
     A.div_nx.init((uint32_t)(A.nx < (1LL << 31) ? A.nx : 1));
 }
 
+// Lanes (log2) of the segments a row of `pairs` node pairs is cut into: 32, or
+// 16 or 8 where that leaves at least a tenth (`fifth`: a fifth) of the lanes
+// less without a pair.  Measured with whole warps and cut (GLUPS): FP16 fast
+// 72^3 (36 pairs, 40 lanes instead of 64) 39.5 -> 55.3, 144^3 55.9 -> 64.0, 200^3
+// 57.5 -> 60.9; BF16 strict 72^3 32.8 -> 47.5, 200^3 49.7 -> 57.5; AA FP16 strict
+// 72^3 30.1 -> 38.5, 200^3 47.4 -> 52.2.  At a tenth (100^3) the gain is 0-5 %.
+inline int row_lanes(int pairs, bool fifth) {
+    int best = 5, lanes = (pairs + 31) / 32 * 32;
+    for (int gs = 4; gs >= 3; --gs) {
+        const int w = 1 << gs, n = (pairs + w - 1) / w * w;
+        if (n * 10 <= lanes * (fifth ? 8 : 9)) { best = gs; lanes = n; }
+    }
+    return best;
+}
+// Geometry of the pair kernels; returns the warps of one step.  The forms for
+// cut rows of three kinds of launch are much slower warp for warp than those for
+// whole-warp segments.  The driven cavity's odd AA step (waves) and launches with
+// an inflow face or an obstacle cut only where whole warps come to more than run
+// at a time (driven AA BF16 40^3 4.62 us/step whole and 5.13 cut, 72^3 11.99 and
+// 10.52), the latter two also for a larger share only (FP16 fast inflow 144x96x96,
+// 72 of 96 lanes, 40.6 -> 43.7 GLUPS; 200x140x140, 104 of 128, 47.1 -> 45.8).
+template <class S, class C>
+long long pair_geometry(SweepArgs<S, C>& A, bool waves, bool obs) {
+    const bool slow = obs || A.bcase == BC_INFLOW;
+    const int pairs = A.l / 2;
+    const long long rows = (long long)A.m * A.n;
+    const long long resident = 148LL * kPairBlocks * (kPairThreads / 32);
+    A.gs = (waves || slow) && rows * ((pairs + 31) / 32) <= resident ? 5 : row_lanes(pairs, slow);
+    A.lmask = (1 << A.gs) - 1;
+    A.nseg = (pairs + A.lmask) >> A.gs;
+    A.div_seg.init((uint32_t)A.nseg);
+    return (A.nseg * rows + (32 >> A.gs) - 1) / (32 >> A.gs);
+}
+
 // True unless the collision can use the shifted, force-free specialisation.
 inline bool generic_collision(const bgk_sweep_params* p) {
     return !(p->cte1 == 1.0 && p->cte0 == 0.0 && p->fx == 0.0 && p->fy == 0.0 && p->fz == 0.0);

@@ -80,10 +80,27 @@ template <class S, class C, int BC, class IDX, int CM, bool OBS> struct Ab2Launc
             sweep_ab2_kernel<S, C, BC, IDX, CM><<<blocks, 256, 0, st>>>(A);
     }
 };
+// True for the pair kernels that have, beside the form for rows cut into
+// segments (SweepArgs::gs), one for whole-warp segments, which is the faster one
+// for those (GLUPS in the cut form and in their own: FP16 fast 256^3 periodic
+// 68.9 and 70.7, inflow 54.0 and 59.1; the driven cavity's odd AA step, BF16
+// 64^3, 42.3 and 44.4 over both steps: its cut form must vote on the wall rows).
+// The others run alike or, the driven cavity's AB sweep, faster in the cut
+// form (FP16 fast 256^3 60.3 -> 64.2).
+constexpr bool whole_form(int bc, bool obs, bool aa) {
+    return obs || bc == BC_INFLOW || (aa ? bc == BC_DRIVEN : bc != BC_DRIVEN);
+}
 template <class S, class C, int BC, class IDX, int CM, bool OBS> struct AbpLaunch {
     static void go(const SweepArgs<S, C>& A, unsigned blocks, cudaStream_t st) {
-        if constexpr (sizeof(S) == 2 && sizeof(C) == 4 && sizeof(IDX) == 4)
-            sweep_abp_kernel<S, C, BC, CM, OBS><<<blocks, kPairThreads, 0, st>>>(A);
+        if constexpr (sizeof(S) == 2 && sizeof(C) == 4 && sizeof(IDX) == 4) {
+            if constexpr (whole_form(BC, OBS, false)) {
+                if (A.gs == 5) {
+                    sweep_abp_kernel<S, C, BC, CM, OBS, false><<<blocks, kPairThreads, 0, st>>>(A);
+                    return;
+                }
+            }
+            sweep_abp_kernel<S, C, BC, CM, OBS, true><<<blocks, kPairThreads, 0, st>>>(A);
+        }
     }
 };
 // True when every node pair (i, i + 1), i odd, is one aligned 32-bit word in
@@ -163,11 +180,9 @@ int launch_sweep(const bgk_sweep_params* p, void* const* a, void* const* b, doub
     const unsigned nb = (unsigned)(mom ? mp.blocks : blocks);
     if constexpr (sizeof(S) == 2 && sizeof(C) == 4) {
         if (g_pair_kernels && mom == nullptr && nelem < (1LL << 31) && pairs_aligned<S>(p, a, b)) {
-            // adjacent node pairs: 64-node segments from i = 1
+            // adjacent node pairs
             SweepArgs<S, C> A2 = A;
-            A2.nseg = (p->l + 63) / 64;
-            A2.div_seg.init((uint32_t)A2.nseg);
-            const long long w2 = (long long)A2.nseg * p->m * p->n;
+            const long long w2 = pair_geometry(A2, false, obs);
             constexpr int wpb = kPairThreads / 32;
             const unsigned nb2 = (unsigned)((w2 + wpb - 1) / wpb);
             switch (p->bcase) {
@@ -461,34 +476,48 @@ void launch_aa_bc(const SweepArgs<S, C>& A, bool odd, long long nelem, unsigned 
     else by_variant<AaEvenLaunch, S, C, BC>(nelem, cm, obs, A, blocks, st);
 }
 
-template <class S, class C, int BC, bool OBS>
+template <class S, class C, int BC, bool OBS, bool CUT>
 void launch_aa_odd_pair_obs(const SweepArgs<S, C>& A, int cm, unsigned blocks, cudaStream_t st) {
     switch (cm) {
-        case CM_STRICT: aa_odd_pair_kernel<S, C, BC, CM_STRICT, OBS><<<blocks, kPairThreads, 0, st>>>(A); break;
+        case CM_STRICT: aa_odd_pair_kernel<S, C, BC, CM_STRICT, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A); break;
         case CM_STRICT_GENERIC:
-            aa_odd_pair_kernel<S, C, BC, CM_STRICT_GENERIC, OBS><<<blocks, kPairThreads, 0, st>>>(A);
+            aa_odd_pair_kernel<S, C, BC, CM_STRICT_GENERIC, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A);
             break;
-        case CM_FAST: aa_odd_pair_kernel<S, C, BC, CM_FAST, OBS><<<blocks, kPairThreads, 0, st>>>(A); break;
-        default: aa_odd_pair_kernel<S, C, BC, CM_FAST_GENERIC, OBS><<<blocks, kPairThreads, 0, st>>>(A); break;
+        case CM_FAST: aa_odd_pair_kernel<S, C, BC, CM_FAST, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A); break;
+        default: aa_odd_pair_kernel<S, C, BC, CM_FAST_GENERIC, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A); break;
     }
 }
 template <class S, class C, int BC>
 void launch_aa_odd_pair(const SweepArgs<S, C>& A, int cm, bool obs, unsigned blocks, cudaStream_t st) {
     if constexpr (sizeof(S) == 2 && sizeof(C) == 4) {
-        if (obs) launch_aa_odd_pair_obs<S, C, BC, true>(A, cm, blocks, st);
-        else launch_aa_odd_pair_obs<S, C, BC, false>(A, cm, blocks, st);
+        if (obs) {
+            if (A.gs == 5) launch_aa_odd_pair_obs<S, C, BC, true, false>(A, cm, blocks, st);
+            else launch_aa_odd_pair_obs<S, C, BC, true, true>(A, cm, blocks, st);
+            return;
+        }
+        if constexpr (whole_form(BC, false, true)) {
+            if (A.gs == 5) { launch_aa_odd_pair_obs<S, C, BC, false, false>(A, cm, blocks, st); return; }
+        }
+        launch_aa_odd_pair_obs<S, C, BC, false, true>(A, cm, blocks, st);
+    }
+}
+template <class S, class C, bool INFLOW, bool OBS, bool CUT>
+void launch_aa_even_pair_cut(const SweepArgs<S, C>& A, int cm, unsigned blocks, cudaStream_t st) {
+    switch (cm) {
+        case CM_STRICT: aa_even_pair_kernel<S, C, CM_STRICT, INFLOW, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A); break;
+        case CM_STRICT_GENERIC:
+            aa_even_pair_kernel<S, C, CM_STRICT_GENERIC, INFLOW, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A);
+            break;
+        case CM_FAST: aa_even_pair_kernel<S, C, CM_FAST, INFLOW, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A); break;
+        default: aa_even_pair_kernel<S, C, CM_FAST_GENERIC, INFLOW, OBS, CUT><<<blocks, kPairThreads, 0, st>>>(A); break;
     }
 }
 template <class S, class C, bool INFLOW, bool OBS>
 void launch_aa_even_pair(const SweepArgs<S, C>& A, int cm, unsigned blocks, cudaStream_t st) {
-    switch (cm) {
-        case CM_STRICT: aa_even_pair_kernel<S, C, CM_STRICT, INFLOW, OBS><<<blocks, kPairThreads, 0, st>>>(A); break;
-        case CM_STRICT_GENERIC:
-            aa_even_pair_kernel<S, C, CM_STRICT_GENERIC, INFLOW, OBS><<<blocks, kPairThreads, 0, st>>>(A);
-            break;
-        case CM_FAST: aa_even_pair_kernel<S, C, CM_FAST, INFLOW, OBS><<<blocks, kPairThreads, 0, st>>>(A); break;
-        default: aa_even_pair_kernel<S, C, CM_FAST_GENERIC, INFLOW, OBS><<<blocks, kPairThreads, 0, st>>>(A); break;
+    if constexpr (INFLOW || OBS) {
+        if (A.gs == 5) { launch_aa_even_pair_cut<S, C, INFLOW, OBS, false>(A, cm, blocks, st); return; }
     }
+    launch_aa_even_pair_cut<S, C, INFLOW, OBS, true>(A, cm, blocks, st);
 }
 
 template <class S, class C>
@@ -512,11 +541,10 @@ int launch_aa(const bgk_sweep_params* p, void* const* slots, bool odd, double* m
         if (g_pair_kernels && mom == nullptr && p->bcase != BC_NONE && nelem < (1LL << 31) &&
             pairs_aligned<S>(p, slots, slots)) {
             SweepArgs<S, C> A2 = A;
-            A2.nseg = (p->l + 63) / 64;
-            A2.div_seg.init((uint32_t)A2.nseg);
             constexpr int wpb = kPairThreads / 32;
-            const unsigned nb2 = (unsigned)(((long long)A2.nseg * p->m * p->n + wpb - 1) / wpb);
             const bool obs = A.obs != nullptr, inflow = p->bcase == BC_INFLOW;
+            const unsigned nb2 =
+                (unsigned)((pair_geometry(A2, odd && p->bcase == BC_DRIVEN, obs) + wpb - 1) / wpb);
             if (!odd) {
                 if (inflow) {
                     if (obs) launch_aa_even_pair<S, C, true, true>(A2, cm, nb2, st);

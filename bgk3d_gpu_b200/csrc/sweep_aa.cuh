@@ -116,26 +116,25 @@ __global__ void __launch_bounds__(256, sizeof(C) == 8 ? 3 : 4) aa_even_kernel(co
 // FP32 pairs and writes population p of both nodes as one word into slot
 // opp(p); bit-identical to aa_even_kernel, in either collision mode.  Purely
 // local, so no shuffles.  INFLOW: node l also writes the outflow halo
-// (aa_even_at's rule) from its values just stored.  OBS: a warp whose 64
-// nodes touch the obstacle's box grown by one node advances them node by
-// node with the one-node rules (solid nodes are not updated).  No fused
+// (aa_even_at's rule) from its values just stored.  OBS: a warp with a
+// pair at the obstacle's box grown by one node advances its nodes one by one with the one-node rules (solid nodes are not updated).  No fused
 // moments.
-template <class S, class C, int CM, bool INFLOW, bool OBS>
+template <class S, class C, int CM, bool INFLOW, bool OBS, bool CUT>
 __global__ void __launch_bounds__(kPairThreads, kPairBlocks) aa_even_pair_kernel(const SweepArgs<S, C> P) {
     static_assert(sizeof(S) == 2 && sizeof(C) == 4, "pair step: 16-bit storage, float compute");
     const uint32_t gw = blockIdx.x * (uint32_t)(kPairThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const uint32_t row = P.div_seg.div(gw);
+    const int gs = CUT ? P.gs : 5, lmask = CUT ? P.lmask : 31;
+    const uint32_t sg = CUT ? lane_segment(P, gw) : gw;
+    const uint32_t row = P.div_seg.div(sg);
     if (row >= P.nrows) return;
-    const int seg = (int)(gw - row * (uint32_t)P.nseg);
+    const int seg = (int)(sg - row * (uint32_t)P.nseg);
     const uint32_t kk = P.div_m.div(row);
     const int j = (int)(row - kk * (uint32_t)P.m) + 1;
     const int k = (int)kk + 1;
-    const int i0 = seg * 64 + 2 * lane + 1;
+    const int i0 = 2 * ((seg << gs) + (int)(threadIdx.x & lmask)) + 1;
     if (i0 >= P.l) return;                            // l even: the pair (i0, i0 + 1) is inside
     const int c = (int)P.nx * j + (int)P.nxy * k + i0;
-    if (OBS && P.obs != nullptr && j >= P.jmin - 1 && j <= P.jmax + 1 && k >= P.kmin - 1 && k <= P.kmax + 1 &&
-        seg * 64 + 64 >= P.imin - 1 && seg * 64 + 1 <= P.imax + 1) {
+    if (OBS && P.obs != nullptr && (CUT ? __any_sync(__activemask(), near_box<CUT>(P, seg, i0, j, k)) : near_box<CUT>(P, seg, i0, j, k))) {
         double m5[5];
         aa_even_at<S, C, INFLOW ? BC_INFLOW : BC_NONE, int, CM, true, false>(P, i0, j, k, c, m5);
         aa_even_at<S, C, INFLOW ? BC_INFLOW : BC_NONE, int, CM, true, false>(P, i0 + 1, j, k, c + 1, m5);
@@ -304,13 +303,13 @@ __global__ void __launch_bounds__(256, sizeof(C) == 8 ? 3 : 4) aa_odd_kernel(con
 // The pairs of one warp of aa_odd_pair_kernel in row (j, k), lane's pair at
 // node ia (element c).  WALLS = false: the row lies on no y or z wall (the
 // driven cavity's inner rows), whose tests and lid term are compiled out.
-template <class S, class C, int BC, int CM, bool WALLS>
-__device__ __forceinline__ void aa_odd_pair_row(const SweepArgs<S, C>& P, int j, int k, int lane, int ia, bool valid,
-                                                int c) {
+template <class S, class C, int BC, int CM, bool WALLS, bool CUT>
+__device__ __forceinline__ void aa_odd_pair_row(const SweepArgs<S, C>& P, int j, int k, int ia, bool valid, int c) {
     typedef Faces<BC> F;
     const int nx = (int)P.nx, nxy = (int)P.nxy;
     const bool at_lo = ia == 1, at_hi = ia + 1 == P.l;
-    const bool edge_lo = lane == 0 || at_lo, edge_hi = lane == 31 || at_hi;
+    const int lmask = CUT ? P.lmask : 31, sub = threadIdx.x & lmask;
+    const bool edge_lo = sub == 0 || at_lo, edge_hi = sub == lmask || at_hi;
     const int oym = (F::PY && j == 1) ? (P.m - 1) * nx : -nx;
     const int oyp = (F::PY && j == P.m) ? (1 - P.m) * nx : nx;
     const int ozm = (F::PZ && k == 1) ? (P.n - 1) * nxy : -nxy;
@@ -456,9 +455,9 @@ __device__ __forceinline__ void aa_odd_pair_row(const SweepArgs<S, C>& P, int j,
 // node 1 pulls the inflow equilibrium across x = 0 and writes it into its
 // own slots 01..05, its populations leaving through x = 0 are dropped, and
 // node l writes the outflow equilibria of its new state (aa_odd_at's rules).
-// OBS: a warp whose 64 nodes touch the obstacle's box grown by one node
-// advances them node by node with the one-node rules.  Pull: population d of the pair's nodes comes
-// from slot opp(d) of the source row as one 32-bit word, the x-shifted half
+// OBS: a warp with a pair at the obstacle's box grown by one node advances all
+// its nodes one by one with the one-node rules.  Pull:
+// population d of the pair's nodes comes from slot opp(d) of the source row as one 32-bit word, the x-shifted half
 // through a lane shuffle as in sweep_abp_kernel (behind a wall: own slot d).
 // Push: population d of both nodes goes to slot d of the target row; for
 // c_x = +-1 the word at the lane's own pair position holds one value of this
@@ -468,28 +467,30 @@ __device__ __forceinline__ void aa_odd_pair_row(const SweepArgs<S, C>& P, int j,
 // read it (or, within a warp, after the neighbour lane's read through the
 // shuffled data), so the in-place update has no hazard.  Bit-identical to
 // aa_odd_kernel.
-template <class S, class C, int BC, int CM, bool OBS>
+template <class S, class C, int BC, int CM, bool OBS, bool CUT>
 __global__ void __launch_bounds__(kPairThreads, kPairBlocks) aa_odd_pair_kernel(const SweepArgs<S, C> P) {
     static_assert(sizeof(S) == 2 && sizeof(C) == 4, "pair step: 16-bit storage, float compute");
     static_assert(BC == BC_DRIVEN || BC == BC_PERIODIC || BC == BC_CHANNEL || BC == BC_INFLOW,
                   "pair odd step: a boundary case");
     typedef Faces<BC> F;
     const uint32_t gw = blockIdx.x * (uint32_t)(kPairThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const uint32_t row = P.div_seg.div(gw);
-    if (row >= P.nrows) return;                       // whole warp
-    const int seg = (int)(gw - row * (uint32_t)P.nseg);
+    const int gs = CUT ? P.gs : 5, lmask = CUT ? P.lmask : 31;
+    const uint32_t sg = CUT ? lane_segment(P, gw) : gw;
+    uint32_t row = P.div_seg.div(sg);
+    const bool inside = row < P.nrows;
+    if (CUT ? !__any_sync(0xffffffffu, inside) : !inside) return;   // whole warp
+    if (!inside) row = P.nrows - 1;
+    const int seg = (int)(sg - row * (uint32_t)P.nseg);
     const uint32_t kk = P.div_m.div(row);
     const int j = (int)(row - kk * (uint32_t)P.m) + 1;
     const int k = (int)kk + 1;
-    const int i0 = seg * 64 + 2 * lane + 1;
-    const bool valid = i0 < P.l;                      // l even: the pair (i0, i0 + 1) is inside
+    const int i0 = 2 * ((seg << gs) + (int)(threadIdx.x & lmask)) + 1;
+    const bool valid = inside && i0 < P.l;            // l even: the pair (i0, i0 + 1) is inside
     const int ia = valid ? i0 : P.l - 1;              // other lanes read a valid pair, store nothing
     const int nx = (int)P.nx, nxy = (int)P.nxy;
     const int c = nx * j + nxy * k + ia;
-    if (OBS && P.obs != nullptr && j >= P.jmin - 1 && j <= P.jmax + 1 && k >= P.kmin - 1 && k <= P.kmax + 1 &&
-        seg * 64 + 64 >= P.imin - 1 && seg * 64 + 1 <= P.imax + 1) {
-        // the warp's 64 nodes touch the obstacle's box grown by one node:
+    if (OBS && P.obs != nullptr && (CUT ? __any_sync(0xffffffffu, near_box<CUT>(P, seg, ia, j, k)) : near_box<CUT>(P, seg, ia, j, k))) {
+        // a pair of the warp touches the obstacle's box grown by one node:
         // node by node with the one-node rules (each node reads and writes
         // only slots no other node touches, so the order does not matter)
         double m5[5];
@@ -499,10 +500,11 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocks) aa_odd_pair_kernel(
         }
         return;
     }
-    if (BC != BC_DRIVEN || j == 1 || j == P.m || k == 1 || k == P.n)
-        aa_odd_pair_row<S, C, BC, CM, true>(P, j, k, lane, ia, valid, c);
+    const bool wall_row = j == 1 || j == P.m || k == 1 || k == P.n;
+    if (BC != BC_DRIVEN || (CUT ? __any_sync(0xffffffffu, wall_row) : wall_row))
+        aa_odd_pair_row<S, C, BC, CM, true, CUT>(P, j, k, ia, valid, c);
     else
-        aa_odd_pair_row<S, C, BC, CM, false>(P, j, k, lane, ia, valid, c);
+        aa_odd_pair_row<S, C, BC, CM, false, CUT>(P, j, k, ia, valid, c);
 }
 
 // Outflow halo in slot form for a freshly loaded Layout E state: halo cell

@@ -52,7 +52,9 @@ template <class S, class C> struct SweepArgs {
     int imin, imax, jmin, jmax, kmin, kmax;
     // launch geometry of the warp-segment mapping
     long long align_base;  // (address of a[0]) / sizeof(S), mod 32
-    int nseg;              // 32-node segments per row
+    int nseg;              // 32-node segments per row (pair kernels: segments of 2^gs pairs)
+    int gs;                // pair kernels: log2 of the lanes of a segment (row_lanes); a warp takes 32 >> gs segments
+    int lmask;             // (1 << gs) - 1
     int nseg_aligned;      // 1 when every row starts on a segment boundary
     uint32_t nrows;        // m * n
     uint32_t nwarps;       // the warps of one step: nseg * nrows, or fwpp * n when flat
@@ -212,6 +214,12 @@ template <class S, class C>
 __device__ __forceinline__ bool in_obstacle_box(const SweepArgs<S, C>& P, int i, int j, int k) {
     return P.obs != nullptr && i >= P.imin - 1 && i <= P.imax + 1 && j >= P.jmin - 1 && j <= P.jmax + 1 &&
            k >= P.kmin - 1 && k <= P.kmax + 1;
+}
+
+// Segment of this lane's group among all segments of the lattice: warp gw's
+// 32 lanes are 32 >> gs groups, one segment each.
+template <class S, class C> __device__ __forceinline__ uint32_t lane_segment(const SweepArgs<S, C>& P, uint32_t gw) {
+    return (gw << (5 - P.gs)) + ((threadIdx.x & 31u) >> P.gs);
 }
 
 // Plane mapping (P.flat): a warp owns 32 consecutive, 32-element aligned
@@ -410,18 +418,31 @@ __global__ void __launch_bounds__(256, 4) sweep_ab2_kernel(const SweepArgs<S, C>
     }
 }
 
+// True when the pair at nodes ia, ia + 1 touches the obstacle's box grown by one node.
+// CUT = false: the same for all pairs of the warp's 64-node segment seg.
+template <bool CUT, class S, class C>
+__device__ __forceinline__ bool near_box(const SweepArgs<S, C>& P, int seg, int ia, int j, int k) {
+    if (!CUT)
+        return j >= P.jmin - 1 && j <= P.jmax + 1 && k >= P.kmin - 1 && k <= P.kmax + 1 &&
+               seg * 64 + 64 >= P.imin - 1 && seg * 64 + 1 <= P.imax + 1;
+    return j >= P.jmin - 1 && j <= P.jmax + 1 && k >= P.kmin - 1 && k <= P.kmax + 1 && ia + 1 >= P.imin - 1 &&
+           ia <= P.imax + 1;
+}
+
 // Adjacent node pairs for the 16-bit kinds on aligned rows of even length:
 // a warp owns 64 consecutive nodes of one row, lane t the pair (i, i + 1)
-// with i = 64 seg + 2t + 1 (i odd, so the pair is one aligned 32-bit word in
+// with i = 64 seg + 2t + 1, or (CUT) 32 >> gs segments of 2^gs pairs, which may
+// belong to several rows: rows of 72 nodes take 5 segments of 8 lanes instead
+// of two warps (i is odd, so the pair is one aligned 32-bit word in
 // every plane).  Per population one 32-bit load fetches the pair at the
-// source row (y/z offsets and their wraps are the same for the whole warp):
+// source row (y/z offsets and their wraps are the same for the whole segment):
 //   c_x =  0: both values;
 //   c_x = +1: node i + 1 takes the low half, node i the high half of lane
 //             t - 1's word (a shuffle);
 //   c_x = -1: node i takes the high half, node i + 1 the low half of lane
 //             t + 1's word.
-// The value the warp does not hold (lane 0's left, lane 31's right
-// neighbour) and the x faces (i = 1, i + 1 = l) are resolved per node by the
+// The value the segment does not hold (its first lane's left, its last lane's
+// right neighbour) and the x faces (i = 1, i + 1 = l) are resolved per node by the
 // one-node rules (gather_at): wrap, bounce-back, inflow equilibrium, outflow
 // halo.  A y/z wall bounces both nodes to their own opposite populations
 // (one aligned load).  The two collisions run as one on packed FP32 pairs
@@ -432,16 +453,17 @@ __global__ void __launch_bounds__(256, 4) sweep_ab2_kernel(const SweepArgs<S, C>
 constexpr int kPairThreads = 128;   // threads per block of sweep_abp_kernel
 constexpr int kPairBlocks = 7;      // resident blocks per SM it is compiled for (72 registers)
 
-// The pairs of one warp in row (j, k): lane's pair starts at node ia; WALLS:
-// the row lies on a y or z wall of the case (compiled separately, so that
-// the rows inside carry no wall logic).
-template <class S, class C, int BC, int CM, bool WALLS>
-__device__ __forceinline__ void abp_row(const SweepArgs<S, C>& P, int j, int k, int lane, int ia, bool valid) {
+// The pair at nodes ia, ia + 1 of row (j, k).  WALLS: the row lies on a y or z
+// wall of the case (compiled separately, so that the rows inside carry no
+// wall logic).
+template <class S, class C, int BC, int CM, bool WALLS, bool CUT>
+__device__ __forceinline__ void abp_row(const SweepArgs<S, C>& P, int j, int k, int ia, bool valid) {
     typedef Faces<BC> F;
     const int nx = (int)P.nx, nxy = (int)P.nxy;
     const int c = nx * j + nxy * k + ia;
     const bool at_lo = ia == 1, at_hi = ia + 1 == P.l;
-    const bool edge_lo = lane == 0 || at_lo, edge_hi = lane == 31 || at_hi;
+    const int lmask = CUT ? P.lmask : 31, sub = threadIdx.x & lmask;
+    const bool edge_lo = sub == 0 || at_lo, edge_hi = sub == lmask || at_hi;
     const int oym = (F::PY && j == 1) ? (P.m - 1) * nx : -nx;
     const int oyp = (F::PY && j == P.m) ? (1 - P.m) * nx : nx;
     const bool zlo = k == 1 && !(P.zhalo & 1), zhi = k == P.n && !(P.zhalo & 2);   // slab faces: halo
@@ -462,7 +484,7 @@ __device__ __forceinline__ void abp_row(const SweepArgs<S, C>& P, int j, int k, 
         if (cy == 1) { off += oym; wl |= wym; } else if (cy == -1) { off += oyp; wl |= wyp; }
         if (cz == 1) { off += ozm; wl |= wzm; } else if (cz == -1) { off += ozp; wl |= wzp; }
         wall[d] = wl;
-        // a y/z wall (same for the whole warp): both nodes bounce back
+        // a y/z wall (same for the whole segment): both nodes bounce back
         const S* src = wl ? P.a[opp_of(d)] + c : P.a[d] + off;
         w[d] = __ldg(reinterpret_cast<const unsigned*>(src));
         if (cx == 1) {
@@ -533,24 +555,26 @@ __device__ __forceinline__ void abp_row(const SweepArgs<S, C>& P, int j, int k, 
     }
 }
 
-template <class S, class C, int BC, int CM, bool OBS>
+template <class S, class C, int BC, int CM, bool OBS, bool CUT>
 __global__ void __launch_bounds__(kPairThreads, kPairBlocks) sweep_abp_kernel(const SweepArgs<S, C> P) {
     static_assert(sizeof(S) == 2 && sizeof(C) == 4, "pair sweep: 16-bit storage, float compute");
     typedef Faces<BC> F;
     const uint32_t gw = blockIdx.x * (uint32_t)(kPairThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const uint32_t row = P.div_seg.div(gw);
-    if (row >= P.nrows) return;                       // whole warp
-    const int seg = (int)(gw - row * (uint32_t)P.nseg);
+    const int gs = CUT ? P.gs : 5, lmask = CUT ? P.lmask : 31;
+    const uint32_t sg = CUT ? lane_segment(P, gw) : gw;
+    uint32_t row = P.div_seg.div(sg);
+    const bool inside = row < P.nrows;
+    if (CUT ? !__any_sync(0xffffffffu, inside) : !inside) return;   // whole warp
+    if (!inside) row = P.nrows - 1;
+    const int seg = (int)(sg - row * (uint32_t)P.nseg);
     const uint32_t kk = P.div_m.div(row);
     const int j = (int)(row - kk * (uint32_t)P.m) + 1;
     const int k = (int)kk + 1;
-    const int i0 = seg * 64 + 2 * lane + 1;
-    const bool valid = i0 < P.l;                      // l even: the pair (i0, i0 + 1) is inside
+    const int i0 = 2 * ((seg << gs) + (int)(threadIdx.x & lmask)) + 1;
+    const bool valid = inside && i0 < P.l;            // l even: the pair (i0, i0 + 1) is inside
     const int ia = valid ? i0 : P.l - 1;              // other lanes read a valid pair, store nothing
-    if (OBS && P.obs != nullptr && j >= P.jmin - 1 && j <= P.jmax + 1 && k >= P.kmin - 1 && k <= P.kmax + 1 &&
-        seg * 64 + 64 >= P.imin - 1 && seg * 64 + 1 <= P.imax + 1) {
-        // the warp's 64 nodes touch the obstacle's box grown by one node:
+    if (OBS && P.obs != nullptr && (CUT ? __any_sync(0xffffffffu, near_box<CUT>(P, seg, ia, j, k)) : near_box<CUT>(P, seg, ia, j, k))) {
+        // a pair of the warp touches the obstacle's box grown by one node:
         // the one-node rules (solid nodes skipped, links into solids bounced)
         double m5[5];
         if (valid) {
@@ -564,8 +588,10 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocks) sweep_abp_kernel(co
     // (spills) and runs slower, so every channel row takes the wall path
     const bool wall_row = (F::WY && (j == 1 || j == P.m)) ||
                           (F::WZ && ((k == 1 && !(P.zhalo & 1)) || (k == P.n && !(P.zhalo & 2))));
-    if (BC != BC_DRIVEN || wall_row) abp_row<S, C, BC, CM, true>(P, j, k, lane, ia, valid);
-    else abp_row<S, C, BC, CM, false>(P, j, k, lane, ia, valid);
+    if (BC != BC_DRIVEN || (CUT ? __any_sync(0xffffffffu, wall_row) : wall_row))
+        abp_row<S, C, BC, CM, true, CUT>(P, j, k, ia, valid);
+    else
+        abp_row<S, C, BC, CM, false, CUT>(P, j, k, ia, valid);
 }
 
 // Outflow halo plane for the inflow case: a10..a14(l+1, j, k) from the

@@ -7,7 +7,7 @@ than L2 for the default size, so no flush is needed).
 
 One JSON line per combination: GLUPS, ms per step, algorithmic HBM GB/s
 (2 x 19 x bytes per value per update) and its fraction of the measured copy
-bandwidth.
+bandwidth (above 1 where a lattice takes two steps per pass over memory).
 """
 from __future__ import annotations
 
@@ -111,7 +111,7 @@ def main(argv=None) -> int:
                             elif pair == "on" and BYTES[kind] == 2:
                                 path = "two-node even step"
                             else:
-                                path = "one-node"
+                                path = "one-node" if pattern == "aa" or tma == "on" else "one-node or two steps per pass"
                             s = time_steps(lat, args.steps, args.warmup)
                             status = lat.L.bgk_lattice_status(lat.h)
                             lat.close()

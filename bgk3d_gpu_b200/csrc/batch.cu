@@ -58,6 +58,12 @@ struct bgk_batch {
     std::vector<char> in_fours;
     std::vector<Group> others;
     std::vector<std::vector<int>> four_branches;   // like branches, over in_fours members, solo members and others
+    // The members' parameters and solid-link tables when the batch was made:
+    // rounds of four run only while they hold, since the groups' launches keep
+    // to the parameters of that time.
+    std::vector<bgk_sweep_params> made;
+    std::vector<const uint32_t*> made_links;
+    bool graph_fours = false;             // the captured graph holds rounds of four
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> ev;          // fork + one join per branch
 };
@@ -278,6 +284,27 @@ int item_step(bgk_batch* B, int item, int par, cudaStream_t st) {
     return group_step(B, B->groups[(size_t)(-1 - item)], par, st);
 }
 
+// The obstacles of the members that take four steps at a time are those the
+// batch was made with.
+bool obstacles_hold(const bgk_batch* B) {
+    for (size_t i = 0; i < B->lats.size(); ++i) {
+        const bgk_lattice* L = B->lats[i];
+        if (B->in_fours[i] && (L->links != B->made_links[i] || L->p.obs != B->made[i].obs)) return false;
+    }
+    return true;
+}
+
+// Rounds of four steps: some member takes them, and all that do are still as
+// the batch was made with.
+bool takes_fours(const bgk_batch* B) {
+    if (B->four_branches.empty() || !obstacles_hold(B)) return false;
+    for (size_t i = 0; i < B->lats.size(); ++i)
+        if (B->in_fours[i] && (!bgk_lat::steps_in_fours(B->lats[i]) ||
+                               std::memcmp(&B->lats[i]->p, &B->made[i], sizeof(bgk_sweep_params)) != 0))
+            return false;
+    return true;
+}
+
 // Four steps of a work item of four_branches from batch parity par (member
 // idx >= 0, or group -1 - idx of the others).
 int item_four(bgk_batch* B, int item, int par, cudaStream_t st) {
@@ -300,7 +327,7 @@ int item_four(bgk_batch* B, int item, int par, cudaStream_t st) {
 // independent lattices, so each branch runs its items' chains of steps
 // (fork / join), and one item's last wave overlaps the others' work.
 int capture_branches(bgk_batch* B) {
-    const bool fours = !B->four_branches.empty();
+    const bool fours = takes_fours(B);
     const std::vector<std::vector<int>>& branches = fours ? B->four_branches : B->branches;
     const size_t G = branches.size();
     while (B->side.size() < G) {
@@ -349,7 +376,7 @@ int batch_one(bgk_batch* B, cudaStream_t st) {
 // nsteps batch steps without the graph: rounds of four where members take
 // them, then single steps.
 int batch_plain(bgk_batch* B, int nsteps, cudaStream_t st) {
-    if (!B->four_branches.empty())
+    if (takes_fours(B))
         for (; nsteps >= 4; nsteps -= 4) {
             for (const std::vector<int>& br : B->four_branches)
                 for (int item : br)
@@ -389,7 +416,8 @@ int build_graph(bgk_batch* B) {
     cudaError_t e = cudaStreamBeginCapture(B->cap, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     int rc = BGK_OK;
-    if (B->chunk > 0 && std::max(B->branches.size(), B->four_branches.size()) > 1) rc = capture_branches(B);
+    B->graph_fours = takes_fours(B);
+    if (B->chunk > 0 && (B->graph_fours ? B->four_branches : B->branches).size() > 1) rc = capture_branches(B);
     else rc = batch_plain(B, kBatchGraphSteps, B->cap);
     e = cudaStreamEndCapture(B->cap, &g);
     B->steps = saved;
@@ -406,6 +434,7 @@ int build_graph(bgk_batch* B) {
 int run_steps(bgk_batch* B, int nsteps, cudaStream_t st) {
     int left = nsteps;
     if (left >= 2 * kBatchGraphSteps) {
+        if (B->graph && B->graph_fours && !obstacles_hold(B)) drop_graph(B);   // it reads the old tables
         if (B->steps & 1) {
             if (int e = batch_one(B, st)) return e;
             --left;
@@ -461,7 +490,11 @@ int bgk_batch_create(bgk_lattice* const* lats, int count, bgk_batch** out) {
         if (L->desc.bcase == BGK_BC_INFLOW) B->inflow.push_back(i);
     }
     B->ntiles = begin[count];
-    for (int i = 0; i < count; ++i) B->expect.push_back(lats[i]->steps);
+    for (int i = 0; i < count; ++i) {
+        B->expect.push_back(lats[i]->steps);
+        B->made.push_back(lats[i]->p);
+        B->made_links.push_back(lats[i]->links);
+    }
     record_base(B);
     int rc = dev_alloc(reinterpret_cast<void**>(&B->desc), host.size(), false, "batch descriptors");
     if (!rc) rc = dev_alloc(reinterpret_cast<void**>(&B->tile_begin), begin.size() * sizeof(uint32_t), false, "tile table");

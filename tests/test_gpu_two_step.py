@@ -100,3 +100,28 @@ def test_batch_members_that_take_two_steps_per_launch(steps):
     batch.close()
     for lat in lats[True] + lats[False]:
         lat.close()
+
+
+def test_batch_member_changed_after_the_batch_was_made():
+    """Groups keep to the parameters their members had when the batch was made;
+    a member that would take four steps at a time does the same, whether the
+    steps run in rounds of four or one by one."""
+    from bgk3d_gpu_b200.lattice import Batch, Lattice
+    l, m, n = 133, 97, 49
+    st0 = random_state(l, m, n, 1, seed=3)
+    out = []
+    for calls in ((7,), (1,) * 7):
+        lats = [Lattice(l, m, n, kind=1, bcase=BCASE["periodic"], omega=OMEGA) for _ in range(2)]
+        for lat in lats:
+            lat.upload(st0)
+        batch = Batch(lats)
+        lats[0].L.bgk_lattice_set_omega(lats[0].h, OMEGA * 0.9)
+        for c in calls:
+            batch.step(c)
+        out.append([lat.download() for lat in lats])
+        batch.close()
+        for lat in lats:
+            lat.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert np.array_equal(out[0][0], out[0][1])

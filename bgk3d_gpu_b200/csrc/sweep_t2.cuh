@@ -235,8 +235,13 @@ __global__ void __launch_bounds__(32 * T2Cfg<C>::WARPS, T2Cfg<C>::BLOCKS) sweep_
     // the tile with its rim reaches x / y faces that wrap, bounce back or carry the inflow and outflow
     const bool xface = i0 <= 2 || i0 + tx >= P.l, yface = j0 <= 2 || j0 + ty >= P.m;
     const bool wraps = (F::PX && xface) || (F::PY && yface), walls = (F::WX && xface) || (F::WY && yface);
-    const bool near_ij = OBS && P.obs != nullptr && i0 - 1 <= P.imax + 1 && i0 + tx >= P.imin - 1 && j0 - 1 <= P.jmax + 1 &&
-                         j0 + ty >= P.jmin - 1;
+    // nodes of the tile or its rim may have links into solid nodes; a rim that
+    // wraps is the node at the axis' other end
+    auto near = [](bool wrapping, int lo, int hi, int ext, int bmin, int bmax) {
+        return (lo <= bmax + 1 && hi >= bmin - 1) || (wrapping && ((lo < 1 && bmax + 1 >= ext) || (hi > ext && bmin - 1 <= 1)));
+    };
+    const bool near_ij = OBS && P.obs != nullptr && near(F::PX, i0 - 1, i0 + tx, P.l, P.imin, P.imax) &&
+                         near(F::PY, j0 - 1, j0 + ty, P.m, P.jmin, P.jmax);
     // plane k of the tile has links that may bounce back
     auto bouncing = [&](int k) {
         return R::BOUNCE && (walls || (F::WZ && (k == 1 || k == P.n)) || (OBS && near_ij && k >= P.kmin - 1 && k <= P.kmax + 1));

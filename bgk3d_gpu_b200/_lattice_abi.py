@@ -41,6 +41,8 @@ def bind_batch(L) -> None:
     L.bgk_batch_get_solo.restype = c_longlong
     L.bgk_batch_groups.argtypes = [c_void_p]
     L.bgk_batch_groups.restype = c_int
+    L.bgk_batch_two_step_members.argtypes = [c_void_p]
+    L.bgk_batch_two_step_members.restype = c_int
     L.bgk_batch_get_config.argtypes = [c_void_p, P_(c_int), P_(c_int)]
     L.bgk_batch_get_config.restype = c_int
     L.bgk_batch_tune.argtypes = [c_void_p, c_int, c_void_p, P_(c_int)]
@@ -80,6 +82,8 @@ def bind(L) -> None:
     L.bgk_lattice_slice.restype = c_int
     L.bgk_lattice_uses_tma.argtypes = [c_void_p]
     L.bgk_lattice_uses_tma.restype = c_int
+    L.bgk_lattice_uses_two_steps.argtypes = [c_void_p]
+    L.bgk_lattice_uses_two_steps.restype = c_int
     L.bgk_set_tma_kernels.argtypes = [c_int]
     L.bgk_set_tma_kernels.restype = c_int
     L.bgk_lattice_status.argtypes = [c_void_p]

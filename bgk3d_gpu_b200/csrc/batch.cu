@@ -592,6 +592,11 @@ int bgk_batch_groups(const bgk_batch* B) {
     return B ? (int)(B->chunk > 0 ? B->groups.size() + B->solo.size() : 1) : -1;
 }
 
+int bgk_batch_two_step_members(const bgk_batch* B) {
+    if (!B) return -1;
+    return takes_fours(B) ? (int)std::count(B->in_fours.begin(), B->in_fours.end(), 1) : 0;
+}
+
 int bgk_batch_get_config(const bgk_batch* B, int* sub, int* bpsm) {
     if (!B) return set_error(BGK_ERR_ARG, "null batch");
     if (sub) *sub = B->sub;

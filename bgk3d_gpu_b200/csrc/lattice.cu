@@ -143,7 +143,7 @@ void drop_links(bgk_lattice* L) {
 
 // nsteps steps without the graph.
 int plain_steps(bgk_lattice* L, int nsteps, cudaStream_t st) {
-    if (bgk_lat::steps_in_fours(L) && !(L->tma_ok && g_tma_kernels))
+    if (bgk_lattice_uses_two_steps(L))
         for (; nsteps >= 4; nsteps -= 4) {
             if (int e = bgk_lat::four_steps(L, L->a, L->b, L->outflow_fresh, st)) return e;
             L->outflow_fresh = L->p.bcase == BC_INFLOW;
@@ -406,6 +406,10 @@ int bgk_lattice_uses_tma(const bgk_lattice* L) {
     if (!L) return 0;
     const bool has_obs = L->p.obs && L->p.imin <= L->p.imax;
     return (L->tma_ok && g_tma_kernels && !has_obs && !L->p.zhalo) ? 1 : 0;
+}
+
+int bgk_lattice_uses_two_steps(const bgk_lattice* L) {
+    return (L && bgk_lat::steps_in_fours(L) && !(L->tma_ok && g_tma_kernels)) ? 1 : 0;
 }
 
 int bgk_lattice_set_zhalo(bgk_lattice* L, int flags) {

@@ -303,6 +303,11 @@ class Lattice:
     def step(self, nsteps=1) -> None:
         check(self.L.bgk_lattice_step(self.h, int(nsteps), self._stream()), "bgk_lattice_step")
 
+    @property
+    def uses_two_steps(self) -> bool:
+        """True if runs of four steps go as two launches of two steps each."""
+        return bool(self.L.bgk_lattice_uses_two_steps(self.h))
+
     def prepare(self) -> None:
         """Capture the step graph now (nothing runs), so that the first long
         step run starts without the capture."""
@@ -406,6 +411,11 @@ class Batch:
     def groups(self) -> int:
         """Launches per step of the grouped form (groups + solo members)."""
         return int(self.L.bgk_batch_groups(self.h))
+
+    @property
+    def two_step_members(self) -> int:
+        """Members whose steps run four at a time (two launches of two steps each)."""
+        return int(self.L.bgk_batch_two_step_members(self.h))
 
     @property
     def solo(self) -> int:

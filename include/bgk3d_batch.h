@@ -59,6 +59,10 @@ int bgk_batch_set_solo(bgk_batch* batch, long long min_nodes);
 long long bgk_batch_get_solo(const bgk_batch* batch);
 int bgk_batch_groups(const bgk_batch* batch);
 
+/* Members whose steps run four at a time, as two launches of two steps each
+   (bgk_lattice_uses_two_steps), in the batch's present form. */
+int bgk_batch_two_step_members(const bgk_batch* batch);
+
 /* Tile queue parameters: tiles taken per queue access (1..16) and resident
    blocks per SM of the persistent grid (1..8); blocks_per_sm = 0 selects the
    non-persistent form, one block per tile.  Used when the chunk size is 0. */

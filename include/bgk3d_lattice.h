@@ -188,8 +188,11 @@ int bgk_lattice_slice(const bgk_lattice* lat, int plane, int index, float* out_d
    bgk_lattice_status: BGK_ERR_CUDA when a TMA sweep gave up waiting for its
    copies (about one second; the kernel then returns and the state is
    undefined) or a two-step launch for its block's warps, else BGK_OK;
-   synchronous.  No counterpart in the reference. */
+   synchronous.  bgk_lattice_uses_two_steps: 1 if bgk_lattice_step takes runs
+   of four steps as two launches of two steps each.  No counterpart in the
+   reference. */
 int bgk_lattice_uses_tma(const bgk_lattice* lat);
+int bgk_lattice_uses_two_steps(const bgk_lattice* lat);
 int bgk_set_tma_kernels(int enable);
 int bgk_lattice_status(const bgk_lattice* lat);
 

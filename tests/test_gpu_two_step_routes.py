@@ -1,0 +1,84 @@
+"""Which calls take two steps per launch, and that the launches end without a
+wait that gave up: the tests that compare such runs with single steps say
+nothing where both take single steps."""
+import numpy as np
+import pytest
+
+from _cases import BCASE, OMEGA, random_state, sphere_mask
+
+pytestmark = pytest.mark.gpu
+
+# above the lines of the dispatch, with and without an obstacle
+LARGE = {"periodic": (133, 130, 80), "channel": (101, 170, 100), "driven": (199, 150, 95), "inflow": (150, 131, 101)}
+
+
+def lattice(shape, case, kind=1, sphere=False, state=None, fast=False):
+    from bgk3d_gpu_b200.lattice import Lattice
+    from test_gpu_lattice import lattice_kwargs
+    lat = Lattice(*shape, kind=kind, bcase=BCASE[case], omega=OMEGA, fast=fast, **lattice_kwargs(case))
+    if sphere:
+        l, m, n = shape
+        lat.set_obstacle(sphere_mask(l, m, n, (l / 3, (m + 1) / 2, (n + 1) / 2), min(m, n) / 6))
+    if state is not None:
+        lat.upload(state)
+    return lat
+
+
+def status(lat):
+    return lat.L.bgk_lattice_status(lat.h)
+
+
+@pytest.mark.parametrize("sphere", [False, True])
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("case", sorted(LARGE))
+def test_large_lattices_take_two_steps_per_launch(case, kind, sphere):
+    """... and their states are those of single steps, bit for bit."""
+    shape = LARGE[case]
+    st0 = random_state(*shape, kind, seed=7)
+    a, b = (lattice(shape, case, kind, sphere, st0) for _ in range(2))
+    assert a.uses_two_steps
+    a.step(5)
+    for _ in range(5):
+        b.step(1)
+    assert status(a) == 0
+    assert np.array_equal(a.download().view(np.uint8), b.download().view(np.uint8))
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("case", sorted(LARGE))
+def test_small_in_place_and_16_bit_lattices_take_single_steps(case):
+    from bgk3d_gpu_b200.lattice import Lattice
+    for kind, shape, pattern in [(1, (40, 40, 40), "ab"), (1, LARGE[case], "aa"), (2, LARGE[case], "ab"), (3, LARGE[case], "ab")]:
+        lat = Lattice(*shape, kind=kind, bcase=BCASE[case], omega=OMEGA, pattern=pattern, scale=256.0 if kind == 2 else 1.0)
+        assert not lat.uses_two_steps
+        lat.close()
+
+
+def test_switches_that_turn_two_steps_off():
+    from bgk3d_gpu_b200._lib import lib
+    lat = lattice(LARGE["periodic"], "periodic")
+    assert lat.uses_two_steps
+    lat.set_zhalo(1)
+    assert not lat.uses_two_steps
+    lat.set_zhalo(0)
+    prev = lib().bgk_set_tma_kernels(1)
+    try:
+        assert lat.uses_two_steps != bool(lib().bgk_lattice_uses_tma(lat.h))
+    finally:
+        lib().bgk_set_tma_kernels(prev)
+    lat.close()
+
+
+def test_batches_count_their_two_step_members():
+    from bgk3d_gpu_b200.lattice import Batch
+    lats = [lattice(LARGE["periodic"], "periodic"), lattice((24, 20, 22), "channel"), lattice(LARGE["inflow"], "inflow", sphere=True)]
+    batch = Batch(lats)
+    assert batch.two_step_members == 2
+    batch.step(20)
+    assert [status(lat) for lat in lats] == [0, 0, 0]
+    batch.set_config(2, 4)                       # the tile-queue form takes single steps
+    assert batch.two_step_members == 0
+    batch.close()
+    for lat in lats:
+        lat.close()

@@ -58,11 +58,14 @@ struct bgk_batch {
     std::vector<char> in_fours;
     std::vector<Group> others;
     std::vector<std::vector<int>> four_branches;   // like branches, over in_fours members, solo members and others
-    // The members' parameters and solid-link tables when the batch was made:
-    // rounds of four run only while they hold, since the groups' launches keep
-    // to the parameters of that time.
+    // The members' parameters when the batch was made: rounds of four run only
+    // while they hold, since the groups' launches keep to the parameters of
+    // that time.
     std::vector<bgk_sweep_params> made;
-    std::vector<const uint32_t*> made_links;
+    // The members' obstacles that the kernel arguments point to
+    // (bgk_lattice::obs_version; the mask's address says nothing, memory is
+    // handed out again).
+    std::vector<long long> obs_version;
     bool graph_fours = false;             // the captured graph holds rounds of four
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> ev;          // fork + one join per branch
@@ -135,6 +138,11 @@ void record_base(bgk_batch* B) {
             B->base_a[19 * i + d] = B->lats[i]->a[d];
             B->base_b[19 * i + d] = B->lats[i]->b[d];
         }
+}
+
+void record_obstacles(bgk_batch* B) {
+    B->obs_version.clear();
+    for (const bgk_lattice* L : B->lats) B->obs_version.push_back(L->obs_version);
 }
 
 // Warp segments of one step of member L (the row mapping of its padded layout).
@@ -284,20 +292,18 @@ int item_step(bgk_batch* B, int item, int par, cudaStream_t st) {
     return group_step(B, B->groups[(size_t)(-1 - item)], par, st);
 }
 
-// The obstacles of the members that take four steps at a time are those the
-// batch was made with.
+// The members' obstacles are those the kernel arguments point to: the masks
+// and tables of earlier ones are freed memory.
 bool obstacles_hold(const bgk_batch* B) {
-    for (size_t i = 0; i < B->lats.size(); ++i) {
-        const bgk_lattice* L = B->lats[i];
-        if (B->in_fours[i] && (L->links != B->made_links[i] || L->p.obs != B->made[i].obs)) return false;
-    }
+    for (size_t i = 0; i < B->lats.size(); ++i)
+        if (B->lats[i]->obs_version != B->obs_version[i]) return false;
     return true;
 }
 
 // Rounds of four steps: some member takes them, and all that do are still as
 // the batch was made with.
 bool takes_fours(const bgk_batch* B) {
-    if (B->four_branches.empty() || !obstacles_hold(B)) return false;
+    if (B->four_branches.empty()) return false;
     for (size_t i = 0; i < B->lats.size(); ++i)
         if (B->in_fours[i] && (!bgk_lat::steps_in_fours(B->lats[i]) ||
                                std::memcmp(&B->lats[i]->p, &B->made[i], sizeof(bgk_sweep_params)) != 0))
@@ -434,7 +440,6 @@ int build_graph(bgk_batch* B) {
 int run_steps(bgk_batch* B, int nsteps, cudaStream_t st) {
     int left = nsteps;
     if (left >= 2 * kBatchGraphSteps) {
-        if (B->graph && B->graph_fours && !obstacles_hold(B)) drop_graph(B);   // it reads the old tables
         if (B->steps & 1) {
             if (int e = batch_one(B, st)) return e;
             --left;
@@ -493,8 +498,8 @@ int bgk_batch_create(bgk_lattice* const* lats, int count, bgk_batch** out) {
     for (int i = 0; i < count; ++i) {
         B->expect.push_back(lats[i]->steps);
         B->made.push_back(lats[i]->p);
-        B->made_links.push_back(lats[i]->links);
     }
+    record_obstacles(B);
     record_base(B);
     int rc = dev_alloc(reinterpret_cast<void**>(&B->desc), host.size(), false, "batch descriptors");
     if (!rc) rc = dev_alloc(reinterpret_cast<void**>(&B->tile_begin), begin.size() * sizeof(uint32_t), false, "tile table");
@@ -524,11 +529,15 @@ int bgk_batch_resync(bgk_batch* B) {
         host.insert(host.end(), tmp, tmp + rec);
         B->expect[i] = L->steps;
     }
-    cudaError_t e = cudaMemcpy(B->desc, host.data(), host.size(), cudaMemcpyHostToDevice);
+    // launches of earlier steps, on any stream, may still read the arguments
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(B->desc, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "resync: %s", cudaGetErrorString(e));
     record_base(B);
     B->steps = 0;
-    return build_groups(B);
+    if (int rc = build_groups(B)) return rc;
+    record_obstacles(B);
+    return BGK_OK;
 }
 
 int bgk_batch_destroy(bgk_batch* B) {
@@ -550,6 +559,8 @@ int bgk_batch_step(bgk_batch* B, int nsteps, void* stream) {
     for (size_t i = 0; i < B->lats.size(); ++i)
         if (B->lats[i]->steps != B->expect[i])
             return set_error(BGK_ERR_STATE, "member %zu was stepped or reloaded outside the batch; create the batch again", i);
+    if (!obstacles_hold(B))
+        if (int e = bgk_batch_resync(B)) return e;
     const long long before = B->steps;
     const int rc = run_steps(B, nsteps, (cudaStream_t)stream);
     sync_members(B, B->steps - before);

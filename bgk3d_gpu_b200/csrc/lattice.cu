@@ -475,6 +475,7 @@ int bgk_lattice_destroy(bgk_lattice* L) {
 int bgk_lattice_set_sphere(bgk_lattice* L, double cx, double cy, double cz, double r2) {
     if (!L) return set_error(BGK_ERR_ARG, "null lattice");
     drop_graph(L);
+    ++L->obs_version;
     drop_links(L);
     dev_free(L->obs_dev);
     L->obs_dev = nullptr;
@@ -512,6 +513,7 @@ int bgk_lattice_set_sphere(bgk_lattice* L, double cx, double cy, double cz, doub
 int bgk_lattice_set_obstacle(bgk_lattice* L, const int32_t* obs) {
     if (!L) return set_error(BGK_ERR_ARG, "null lattice");
     drop_graph(L);
+    ++L->obs_version;
     drop_links(L);
     dev_free(L->obs_dev);
     L->obs_dev = nullptr;

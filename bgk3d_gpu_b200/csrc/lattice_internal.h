@@ -21,6 +21,7 @@ struct bgk_lattice {
     void* rest = nullptr;        // AB, large: a second array of population 19 at element (0,0,0) (two-step sweep), or null
     uint32_t* links = nullptr;   // with an obstacle: its table of solid links (two-step sweep), or null
     int32_t* obs_dev = nullptr;
+    long long obs_version = 0;   // raised whenever the obstacle's mask and table are replaced
     long long steps = 0;
     double* ws = nullptr;
     size_t ws_bytes = 0;

@@ -37,7 +37,10 @@ int bgk_batch_create(bgk_lattice* const* lattices, int count, bgk_batch** out);
 int bgk_batch_destroy(bgk_batch* batch);
 
 /* Advance every member nsteps steps, stream-ordered.  BGK_ERR_STATE if a
-   member was stepped or reloaded on its own since the batch last ran. */
+   member was stepped or reloaded on its own since the batch last ran.  A
+   member whose obstacle was set anew since then is taken over with it (as
+   bgk_batch_resync does, which waits for the device); other parameters set on
+   a member take effect at the next resync. */
 int bgk_batch_step(bgk_batch* batch, int nsteps, void* stream);
 
 /* Accept the members' current states after they were loaded or stepped on

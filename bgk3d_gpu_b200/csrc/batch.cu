@@ -58,9 +58,8 @@ struct bgk_batch {
     std::vector<char> in_fours;
     std::vector<Group> others;
     std::vector<std::vector<int>> four_branches;   // like branches, over in_fours members, solo members and others
-    // The members' parameters when the batch was made: rounds of four run only
-    // while they hold, since the groups' launches keep to the parameters of
-    // that time.
+    // The members' parameters that the kernel arguments were made from; rounds
+    // of four keep to them as the groups' launches do.
     std::vector<bgk_sweep_params> made;
     // The members' obstacles that the kernel arguments point to
     // (bgk_lattice::obs_version; the mask's address says nothing, memory is
@@ -140,9 +139,15 @@ void record_base(bgk_batch* B) {
         }
 }
 
-void record_obstacles(bgk_batch* B) {
+// What the kernel arguments are made from.
+void record_members(bgk_batch* B) {
+    record_base(B);
+    B->made.clear();
     B->obs_version.clear();
-    for (const bgk_lattice* L : B->lats) B->obs_version.push_back(L->obs_version);
+    for (const bgk_lattice* L : B->lats) {
+        B->made.push_back(L->p);
+        B->obs_version.push_back(L->obs_version);
+    }
 }
 
 // Warp segments of one step of member L (the row mapping of its padded layout).
@@ -165,6 +170,8 @@ constexpr int kBranches = 8;
 long long member_nodes(const bgk_batch* B, int i) {
     return B->lats[i]->desc.l * (long long)B->lats[i]->desc.m * B->lats[i]->desc.n;
 }
+
+bool is_solo(const bgk_batch* B, int i) { return std::find(B->solo.begin(), B->solo.end(), i) != B->solo.end(); }
 
 // Groups, solo members, graph branches and the chunk table of the grouped
 // form for the current chunk size and solo threshold.
@@ -219,8 +226,8 @@ int build_groups(bgk_batch* B) {
     if (B->chunk <= 0) return BGK_OK;
     std::vector<int> alone;
     for (size_t i = 0; i < B->lats.size(); ++i) {
-        B->in_fours[i] = bgk_lat::steps_in_fours(B->lats[i]) ? 1 : 0;
-        if (B->in_fours[i] || std::find(B->solo.begin(), B->solo.end(), (int)i) != B->solo.end()) alone.push_back((int)i);
+        B->in_fours[i] = bgk_lat::steps_in_fours(B->lats[i], &B->made[i]) ? 1 : 0;
+        if (B->in_fours[i] || is_solo(B, (int)i)) alone.push_back((int)i);
     }
     for (const bgk_batch::Group& g : B->groups) {
         bgk_batch::Group o = g;
@@ -300,26 +307,24 @@ bool obstacles_hold(const bgk_batch* B) {
     return true;
 }
 
-// Rounds of four steps: some member takes them, and all that do are still as
-// the batch was made with.
-bool takes_fours(const bgk_batch* B) {
-    if (B->four_branches.empty()) return false;
-    for (size_t i = 0; i < B->lats.size(); ++i)
-        if (B->in_fours[i] && (!bgk_lat::steps_in_fours(B->lats[i]) ||
-                               std::memcmp(&B->lats[i]->p, &B->made[i], sizeof(bgk_sweep_params)) != 0))
-            return false;
-    return true;
-}
+// Rounds of four steps: some member takes them.
+bool takes_fours(const bgk_batch* B) { return !B->four_branches.empty(); }
 
 // Four steps of a work item of four_branches from batch parity par (member
-// idx >= 0, or group -1 - idx of the others).
+// idx >= 0, or group -1 - idx of the others).  The parameters are those its
+// single steps run with: a solo member's own, a group member's as of the
+// kernel arguments.
 int item_four(bgk_batch* B, int item, int par, cudaStream_t st) {
     if (item >= 0 && B->in_fours[(size_t)item]) {
-        void* a[19];
-        void* b[19];
-        member_arrays(B, (size_t)item, par, a);
-        member_arrays(B, (size_t)item, par ^ 1, b);
-        return bgk_lat::four_steps(B->lats[(size_t)item], a, b, false, st);
+        const bgk_lattice* L = B->lats[(size_t)item];
+        const bgk_sweep_params* p = is_solo(B, item) ? &L->p : &B->made[(size_t)item];
+        if (bgk_lat::steps_in_fours(L, p)) {
+            void* a[19];
+            void* b[19];
+            member_arrays(B, (size_t)item, par, a);
+            member_arrays(B, (size_t)item, par ^ 1, b);
+            return bgk_lat::four_steps(L, p, a, b, false, st);
+        }
     }
     for (int s = 0; s < 4; ++s) {
         const int e = item >= 0 ? member_step(B, item, par ^ (s & 1), st)
@@ -495,12 +500,8 @@ int bgk_batch_create(bgk_lattice* const* lats, int count, bgk_batch** out) {
         if (L->desc.bcase == BGK_BC_INFLOW) B->inflow.push_back(i);
     }
     B->ntiles = begin[count];
-    for (int i = 0; i < count; ++i) {
-        B->expect.push_back(lats[i]->steps);
-        B->made.push_back(lats[i]->p);
-    }
-    record_obstacles(B);
-    record_base(B);
+    for (int i = 0; i < count; ++i) B->expect.push_back(lats[i]->steps);
+    record_members(B);
     int rc = dev_alloc(reinterpret_cast<void**>(&B->desc), host.size(), false, "batch descriptors");
     if (!rc) rc = dev_alloc(reinterpret_cast<void**>(&B->tile_begin), begin.size() * sizeof(uint32_t), false, "tile table");
     if (!rc) rc = dev_alloc(reinterpret_cast<void**>(&B->counter), 2 * sizeof(unsigned), true, "tile counter");
@@ -533,10 +534,12 @@ int bgk_batch_resync(bgk_batch* B) {
     cudaError_t e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(B->desc, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return set_error(BGK_ERR_CUDA, "resync: %s", cudaGetErrorString(e));
-    record_base(B);
     B->steps = 0;
-    if (int rc = build_groups(B)) return rc;
-    record_obstacles(B);
+    record_members(B);
+    if (int rc = build_groups(B)) {
+        B->obs_version[0] = -1;   // the next step tries again
+        return rc;
+    }
     return BGK_OK;
 }
 
@@ -605,7 +608,7 @@ int bgk_batch_groups(const bgk_batch* B) {
 
 int bgk_batch_two_step_members(const bgk_batch* B) {
     if (!B) return -1;
-    return takes_fours(B) ? (int)std::count(B->in_fours.begin(), B->in_fours.end(), 1) : 0;
+    return (int)std::count(B->in_fours.begin(), B->in_fours.end(), 1);
 }
 
 int bgk_batch_get_config(const bgk_batch* B, int* sub, int* bpsm) {

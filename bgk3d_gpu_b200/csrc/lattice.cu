@@ -145,7 +145,7 @@ void drop_links(bgk_lattice* L) {
 int plain_steps(bgk_lattice* L, int nsteps, cudaStream_t st) {
     if (bgk_lattice_uses_two_steps(L))
         for (; nsteps >= 4; nsteps -= 4) {
-            if (int e = bgk_lat::four_steps(L, L->a, L->b, L->outflow_fresh, st)) return e;
+            if (int e = bgk_lat::four_steps(L, &L->p, L->a, L->b, L->outflow_fresh, st)) return e;
             L->outflow_fresh = L->p.bcase == BC_INFLOW;
             L->steps += 4;
         }
@@ -279,25 +279,27 @@ int tma_step(bgk_lattice* L, cudaStream_t st) {
 }  // namespace
 
 namespace bgk_lat {
-static int two_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st) {
-    switch (L->p.kind) {
-        case K_F64: return launch_sweep_t2<double, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
-        case K_F32: return launch_sweep_t2<float, float>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
-        case K_F32_F64: return launch_sweep_t2<float, double>(&L->p, a, b, L->links, L->err, outflow_fresh, st);
+static int two_steps(const bgk_lattice* L, const bgk_sweep_params* p, void* const* a, void* const* b, bool outflow_fresh,
+                     cudaStream_t st) {
+    switch (p->kind) {
+        case K_F64: return launch_sweep_t2<double, double>(p, a, b, L->links, L->err, outflow_fresh, st);
+        case K_F32: return launch_sweep_t2<float, float>(p, a, b, L->links, L->err, outflow_fresh, st);
+        case K_F32_F64: return launch_sweep_t2<float, double>(p, a, b, L->links, L->err, outflow_fresh, st);
     }
     return set_error(BGK_ERR_UNSUPPORTED, "two-step sweep: 4- and 8-byte kinds");
 }
 
-bool steps_in_fours(const bgk_lattice* L) {
-    const bool has_obs = L->p.obs && L->p.imin <= L->p.imax;
-    return L->rest && (!has_obs || L->links) && !L->p.zhalo;
+bool steps_in_fours(const bgk_lattice* L, const bgk_sweep_params* p) {
+    const bool has_obs = p->obs && p->imin <= p->imax;
+    return L->rest && (!has_obs || L->links) && !p->zhalo;
 }
 
-int four_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st) {
+int four_steps(const bgk_lattice* L, const bgk_sweep_params* p, void* const* a, void* const* b, bool outflow_fresh,
+               cudaStream_t st) {
     void* t[19];
     for (int d = 0; d < 19; ++d) t[d] = d < 18 ? b[d] : L->rest;
-    if (int e = two_steps(L, a, t, outflow_fresh, st)) return e;
-    return two_steps(L, t, a, true, st);
+    if (int e = two_steps(L, p, a, t, outflow_fresh, st)) return e;
+    return two_steps(L, p, t, a, true, st);
 }
 
 void observable(const bgk_lattice* L, void** out) {
@@ -409,7 +411,7 @@ int bgk_lattice_uses_tma(const bgk_lattice* L) {
 }
 
 int bgk_lattice_uses_two_steps(const bgk_lattice* L) {
-    return (L && bgk_lat::steps_in_fours(L) && !(L->tma_ok && g_tma_kernels)) ? 1 : 0;
+    return (L && bgk_lat::steps_in_fours(L, &L->p) && !(L->tma_ok && g_tma_kernels)) ? 1 : 0;
 }
 
 int bgk_lattice_set_zhalo(bgk_lattice* L, int flags) {

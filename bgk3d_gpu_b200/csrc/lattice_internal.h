@@ -43,16 +43,17 @@ struct bgk_lattice {
 // Shared by the lattice's host-transfer paths (lattice.cu, lattice_io.cu) and
 // the batched stepper.
 namespace bgk_lat {
-// True when the lattice's steps run four at a time (AB, arrays that outgrow
-// L2, rest population's second array and obstacle table in place).
-bool steps_in_fours(const bgk_lattice* L);
-// Four steps as two two-step launches a -> b -> a.  The arrays end as four
+// True when the lattice's steps with the parameters p run four at a time (AB,
+// arrays that outgrow L2, rest population's second array and obstacle table
+// in place).
+bool steps_in_fours(const bgk_lattice* L, const bgk_sweep_params* p);
+// Four steps with the parameters p as two two-step launches a -> b -> a.  The arrays end as four
 // single steps leave them: a holds the state, and neither the halo nor the
 // solid nodes of either set are written (an inflow lattice's outflow plane
 // is, by both).  The rest population, which single steps update in place,
 // passes through L->rest.  outflow_fresh: a's outflow plane needs no pre-pass
 // (it needs none afterwards either).
-int four_steps(const bgk_lattice* L, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st);
+int four_steps(const bgk_lattice* L, const bgk_sweep_params* p, void* const* a, void* const* b, bool outflow_fresh, cudaStream_t st);
 // Device arrays holding populations 01..19 of the observable state.
 void observable(const bgk_lattice* L, void** out);
 // Reset the pointer arrangement to the base planes and return the arrays a

@@ -75,7 +75,10 @@ int bgk_trim_memory(void);
 
 /* Obstacle mask obs_host[l*m*n] (i fastest, 1 = solid, SRC/build.obs.F90
    convention); copied to the device, bounding box computed here.  Must stay
-   one node inside the lattice.  NULL removes the obstacle. */
+   one node inside the lattice.  NULL removes the obstacle.  Steps neither
+   read nor write solid nodes; an obstacle set between steps leaves in the
+   nodes it covers what either set of arrays held, the current state or one of
+   the two before it. */
 int bgk_lattice_set_obstacle(bgk_lattice* lat, const int32_t* obs_host);
 
 /* Solid sphere obstacle built on the device: nodes with (i - cx)^2 +
@@ -135,8 +138,8 @@ long long bgk_io_set_subrecord_limit(long long bytes);
    Runs of 32 or more steps replay a captured 16-step CUDA graph (captured on
    the first such run unless bgk_lattice_prepare captured it before).  AB
    lattices of the 4- and 8-byte kinds whose arrays outgrow the L2 cache take
-   four steps at a time as two launches of two steps each; the result is bit
-   for bit that of single steps. */
+   four steps at a time as two launches of two steps each; the state outside
+   solid nodes is bit for bit that of single steps. */
 int bgk_lattice_step(bgk_lattice* lat, int nsteps, void* stream);
 
 /* Capture the 16-step CUDA graph of bgk_lattice_step now, without running

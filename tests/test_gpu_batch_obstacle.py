@@ -1,7 +1,10 @@
 """Obstacles replaced between the steps of a batch: the batch goes on with the
 new ones, in its groups and in its members that take two steps per launch,
 although the old masks' memory is freed and may be handed out again at the
-same address.  Every member's state is that of the lattice stepped alone."""
+same address.  Every member's state is that of the lattice stepped alone, in every
+node outside the last obstacle (the nodes that it covers keep what they held in
+either of the lattice's two sets of arrays, whose other set is one step back
+after a single step and two after two steps per launch)."""
 import numpy as np
 import pytest
 
@@ -36,8 +39,7 @@ def replace(lats, part, how):
         elif how == "sphere":
             lat.set_sphere(*sphere(shape, part))
         else:
-            c, r2 = sphere(shape, part)
-            lat.set_obstacle(sphere_mask(*shape, c, r2 ** 0.5))
+            lat.set_obstacle(sphere_mask(*shape, *sphere(shape, part)))
 
 
 @pytest.mark.parametrize("retained", [0, 1 << 30])
@@ -63,7 +65,10 @@ def test_obstacles_replaced_between_runs(how, resync, retained):
                     batch.resync()
         for (case, shape), a, b in zip(MEMBERS, alone, lats):
             assert b.L.bgk_lattice_status(b.h) == 0
-            assert np.array_equal(a.download(), b.download()), f"{case} {shape}"
+            same = a.download() == b.download()
+            if how != "none":
+                same[:, 1:-1, 1:-1, 1:-1] |= sphere_mask(*shape, *sphere(shape, 0.4)) == 1
+            assert same.all(), f"{case} {shape}"
         batch.close()
         for lat in alone + lats:
             lat.close()

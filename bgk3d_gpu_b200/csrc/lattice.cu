@@ -105,24 +105,56 @@ int one_step(bgk_lattice* L, cudaStream_t st, double* mom = nullptr, double* mom
     return BGK_OK;
 }
 
-// Bytes of a lattice's arrays from which its steps run four at a time, as two
-// launches of two steps each (sweep_t2.cuh): where they outgrow the 126 MB L2.
-// Below that the one-step sweep runs from L2 and the rims cost more than they save
-// (FP32 64^3, 62 MB: 41 GLUPS against 34; FP64 64^3, 124 MB: 26 against 25).
-// Where the line lies depends on the case, whose face and obstacle blocks
-// take longer: periodic 120 MB (FP32 80^3, 127 MB, 35.2 -> 37.4), walls 150 MB
-// (FP32 driven 80^3 34.6 against 30.1; 96^3, 182 MB, 36.6 -> 41.5), inflow 300 MB
-// (FP32 with a sphere 199x83x61, 203 MB, 31.7 against 28.8; 128^3, 400 MB, 34.9
-// -> 36.4).
-size_t two_step_line(int bcase) {
-    return (size_t)(bcase == BC_PERIODIC ? 120 : (bcase == BC_INFLOW ? 300 : 150)) << 20;
+// Where a lattice's steps run four at a time, as two launches of two steps each
+// (sweep_t2.cuh): where that was the faster way at 6279 shapes of 15 MB to 4 GB
+// (l 7 to 256, m : n from 1 : 4 to 4 : 1, 32 to 64 steps through the captured
+// graph, with and without a sphere).  Two lines, both in bytes of all arrays:
+//  * the allocation, padding included, has to outgrow the 126 MB L2, from which
+//    the one-step sweep runs below it: two_step_line;
+//  * so have the 128-byte lines that hold nodes, or MiB as follows.  Below, the
+//    one-step sweep still finds part of its state in L2, and the two-step sweep
+//    has few blocks, whose slowest ends the launch: those at a wall or at an
+//    obstacle.  Two steps per pass ran at 0.74-0.95 of one for FP64 periodic and
+//    driven rows of 17 to 32 nodes below 100 MiB, with a sphere at 0.73-0.98
+//    (FP32 driven, 90-300 MiB) and 0.61-1.0 (FP64 driven, to 300 MiB); from the
+//    lines below it gains.
+// The one-step sweep's warps take 32 nodes of a row, the two-step tiles of FP64
+// arithmetic 16: rows that leave a quarter or more of the former's lanes without
+// a node that the latter's have (l to 16, 33 to 48) gain earlier.  FP32 storage
+// with FP64 arithmetic moves half of FP64's bytes for its instructions, so the
+// rims' second computation costs more than a pass saves (0.66-1.08 of one step
+// per pass, with a sphere 0.54-1.0 at most shapes) but for such rows (1.26x) and
+// inflow lattices of 1000 MiB or more (1.01-1.17x).
+// By the rule 3283 of the 6279 shapes take two steps per pass, at 1.24x on
+// average; 34 of them are slower by more than 3 %, the slowest at 0.88 (before
+// there was the second line 1937 were, the slowest at 0.54).
+constexpr size_t kNever = SIZE_MAX >> 20;
+size_t two_step_line(int bcase) { return bcase == BC_PERIODIC ? 120 : (bcase == BC_INFLOW ? 300 : 150); }
+size_t two_step_node_line(const bgk_sweep_params& p, bool obstacle) {
+    //                          driven, periodic, channel, inflow
+    static const size_t f32[2][4] = {{120, 80, 75, 0}, {400, 160, 200, 0}};
+    static const size_t f64[2][4] = {{125, 100, 110, 0}, {400, 200, 300, 400}};
+    if (p.kind == K_F32) return f32[obstacle][p.bcase];
+    const bool idle = 4 * 16 * ((p.l + 15) / 16) <= 3 * 32 * ((p.l + 31) / 32);
+    if (p.kind == K_F64) {
+        const size_t early = obstacle ? 110 : 80;
+        return idle ? std::min(early, f64[obstacle][p.bcase]) : f64[obstacle][p.bcase];
+    }
+    if (obstacle) return kNever;
+    return idle ? 60 : (p.bcase == BC_INFLOW ? 1000 : kNever);
+}
+// p: a library lattice's parameters; bytes: its arrays.
+bool two_steps_pay(const bgk_sweep_params& p, size_t bytes, bool obstacle) {
+    if (p.kind != K_F64 && p.kind != K_F32 && p.kind != K_F32_F64) return false;
+    const size_t row = ((size_t)p.l * elem_bytes(p.kind) + 127) / 128 * 128;
+    return (bytes >> 20) >= two_step_line(p.bcase) && (37 * row * (size_t)p.m * (size_t)p.n >> 20) >= two_step_node_line(p, obstacle);
 }
 
 // The table of solid links the two-step sweep reads (t2_links_kernel), made
-// for the lattice's current obstacle; without it (no memory left) the lattice
-// takes single steps.
+// for the lattice's current obstacle; without it (no memory left, or two steps
+// per pass do not pay with an obstacle) the lattice takes single steps.
 void make_links(bgk_lattice* L) {
-    if (!L->rest) return;
+    if (!L->rest || !two_steps_pay(L->p, L->bytes, true)) return;
     const bgk_sweep_params& p = L->p;
     const long long nodes = (long long)(p.imax - p.imin + 3) * (p.jmax - p.jmin + 3) * (p.kmax - p.kmin + 3);
     void* buf = nullptr;
@@ -367,7 +399,7 @@ int bgk_lattice_create(const bgk_lattice_desc* d, bgk_lattice** out) {
     // population's second one (two-step sweep, 32-bit byte offsets), in the
     // same block of memory; without room for it, it takes single steps
     const size_t array = (size_t)L->plane * L->es;
-    const bool fours = d->pattern == BGK_PATTERN_AB && L->es >= 4 && L->bytes >= two_step_line(d->bcase) && array < (1ULL << 32);
+    const bool fours = d->pattern == BGK_PATTERN_AB && two_steps_pay(L->p, L->bytes, false) && array < (1ULL << 32);
     int rc = fours ? dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes + array, true, "lattice") : BGK_ERR_NOMEM;
     if (rc == BGK_OK) L->rest = L->base + L->bytes + (size_t)(L->shift + L->origin) * L->es;
     else rc = dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes, true, "lattice");

@@ -9,7 +9,7 @@ from _cases import BCASE, OMEGA, random_state
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = {"periodic": (133, 97, 49), "channel": (101, 131, 67), "inflow": (150, 131, 101), "driven": (199, 83, 61)}
+SHAPES = {"periodic": (133, 130, 80), "channel": (101, 170, 100), "inflow": (150, 131, 101), "driven": (199, 150, 95)}
 # where the obstacle's box lies along x, y, z: -1 starts at node 2, +1 ends at the last node but one, 0 inside
 PLACES = [(-1, 0, 0), (1, 0, 0), (0, -1, 0), (0, 1, 0), (0, 0, -1), (0, 0, 1),
           (-1, -1, 0), (1, 1, 0), (-1, 1, -1), (1, -1, 1), (1, 1, 1), (-1, -1, -1)]
@@ -35,6 +35,7 @@ def run(shape, kind, case, calls, obs=None, fast=False):
     lat = Lattice(*shape, kind=kind, bcase=BCASE[case], omega=OMEGA, fast=fast, **lattice_kwargs(case))
     if obs is not None:
         lat.set_obstacle(obs)
+    assert lat.uses_two_steps or kind == 4
     lat.upload(random_state(*shape, kind, seed=shape[0] + kind))
     for c in calls:
         lat.step(c)

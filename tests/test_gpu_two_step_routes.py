@@ -82,3 +82,40 @@ def test_batches_count_their_two_step_members():
     batch.close()
     for lat in lats:
         lat.close()
+
+
+# shapes on both sides of the lines: (kind, case, shape, sphere, two steps per launch); each pair of
+# neighbours differs in what the rule looks at
+LINES = [
+    (0, "periodic", (20, 95, 95), False, False), (0, "periodic", (38, 95, 95), False, True),       # nodes fill L2 or not
+    (0, "driven", (128, 56, 56), False, False), (0, "driven", (128, 80, 80), False, True),
+    (1, "driven", (128, 128, 128), True, False), (1, "driven", (128, 128, 128), False, True),      # obstacle
+    (1, "channel", (101, 131, 67), True, False), (1, "channel", (101, 170, 100), True, True),
+    (1, "periodic", (100, 100, 80), True, False), (1, "periodic", (100, 100, 120), True, True),
+    (0, "driven", (128, 90, 90), True, False), (0, "driven", (128, 128, 128), True, True),
+    (0, "driven", (34, 120, 120), True, True),                                                      # idle lanes
+    (4, "periodic", (128, 128, 128), False, False), (4, "periodic", (40, 150, 110), False, True),   # mixed precision
+    (4, "driven", (128, 200, 200), False, False), (4, "channel", (33, 140, 130), False, True),
+    (4, "periodic", (40, 150, 110), True, False), (4, "inflow", (128, 130, 130), False, False),
+    (4, "inflow", (34, 260, 161), False, True),
+]
+
+
+@pytest.mark.parametrize("kind,case,shape,sphere,two", LINES)
+def test_lines_of_the_dispatch(kind, case, shape, sphere, two):
+    """The route, and the same state as by single steps."""
+    st0 = random_state(*shape, kind, seed=11)
+    a, b = (lattice(shape, case, kind, sphere, st0) for _ in range(2))
+    assert a.uses_two_steps == two
+    a.step(6)
+    for _ in range(6):
+        b.step(1)
+    assert status(a) == 0
+    assert np.array_equal(a.download().view(np.uint8), b.download().view(np.uint8))
+    if sphere:                                   # without it, what the open lattice takes
+        a.set_obstacle(None)
+        c = lattice(shape, case, kind)
+        assert a.uses_two_steps == c.uses_two_steps
+        c.close()
+    a.close()
+    b.close()

@@ -60,6 +60,8 @@ def bind(L) -> None:
     L.bgk_lattice_desc_init.restype = None
     L.bgk_lattice_device_bytes.argtypes = [D]
     L.bgk_lattice_device_bytes.restype = c_size_t
+    L.bgk_lattice_least_bytes.argtypes = [D]
+    L.bgk_lattice_least_bytes.restype = c_size_t
     L.bgk_lattice_create.argtypes = [D, POINTER(c_void_p)]
     L.bgk_lattice_create.restype = c_int
     L.bgk_lattice_destroy.argtypes = [c_void_p]

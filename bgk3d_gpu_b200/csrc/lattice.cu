@@ -130,31 +130,41 @@ int one_step(bgk_lattice* L, cudaStream_t st, double* mom = nullptr, double* mom
 // there was the second line 1937 were, the slowest at 0.54).
 constexpr size_t kNever = SIZE_MAX >> 20;
 size_t two_step_line(int bcase) { return bcase == BC_PERIODIC ? 120 : (bcase == BC_INFLOW ? 300 : 150); }
-size_t two_step_node_line(const bgk_sweep_params& p, bool obstacle) {
+size_t two_step_node_line(int kind, int bcase, int l, bool obstacle) {
     //                          driven, periodic, channel, inflow
     static const size_t f32[2][4] = {{120, 80, 75, 0}, {400, 160, 200, 0}};
     static const size_t f64[2][4] = {{125, 100, 110, 0}, {400, 200, 300, 400}};
-    if (p.kind == K_F32) return f32[obstacle][p.bcase];
-    const bool idle = 4 * 16 * ((p.l + 15) / 16) <= 3 * 32 * ((p.l + 31) / 32);
-    if (p.kind == K_F64) {
+    if (kind == K_F32) return f32[obstacle][bcase];
+    const bool idle = 4 * 16 * ((l + 15LL) / 16) <= 3 * 32 * ((l + 31LL) / 32);
+    if (kind == K_F64) {
         const size_t early = obstacle ? 110 : 80;
-        return idle ? std::min(early, f64[obstacle][p.bcase]) : f64[obstacle][p.bcase];
+        return idle ? std::min(early, f64[obstacle][bcase]) : f64[obstacle][bcase];
     }
     if (obstacle) return kNever;
-    return idle ? 60 : (p.bcase == BC_INFLOW ? 1000 : kNever);
+    return idle ? 60 : (bcase == BC_INFLOW ? 1000 : kNever);
 }
-// p: a library lattice's parameters; bytes: its arrays.
-bool two_steps_pay(const bgk_sweep_params& p, size_t bytes, bool obstacle) {
-    if (p.kind != K_F64 && p.kind != K_F32 && p.kind != K_F32_F64) return false;
-    const size_t row = ((size_t)p.l * elem_bytes(p.kind) + 127) / 128 * 128;
-    return (bytes >> 20) >= two_step_line(p.bcase) && (37 * row * (size_t)p.m * (size_t)p.n >> 20) >= two_step_node_line(p, obstacle);
+// bytes: the arrays of the lattice d describes.
+bool two_steps_pay(const bgk_lattice_desc* d, size_t bytes, bool obstacle) {
+    if (d->kind != K_F64 && d->kind != K_F32 && d->kind != K_F32_F64) return false;
+    if (d->bcase < BC_DRIVEN || d->bcase > BC_INFLOW || d->pattern != BGK_PATTERN_AB) return false;
+    const size_t row = ((size_t)d->l * elem_bytes(d->kind) + 127) / 128 * 128;
+    return (bytes >> 20) >= two_step_line(d->bcase) &&
+           (37 * row * (size_t)d->m * (size_t)d->n >> 20) >= two_step_node_line(d->kind, d->bcase, d->l, obstacle);
+}
+
+// Bytes of one more array, the rest population's second one, which a lattice
+// whose steps run four at a time has behind its arrays (two-step sweep, 32-bit
+// byte offsets); 0 for the others.
+size_t rest_bytes(const bgk_lattice_desc* d) {
+    const size_t array = (size_t)geometry(d).plane * elem_bytes(d->kind);
+    return two_steps_pay(d, array * nplanes(d), false) && array < (1ULL << 32) ? array : 0;
 }
 
 // The table of solid links the two-step sweep reads (t2_links_kernel), made
 // for the lattice's current obstacle; without it (no memory left, or two steps
 // per pass do not pay with an obstacle) the lattice takes single steps.
 void make_links(bgk_lattice* L) {
-    if (!L->rest || !two_steps_pay(L->p, L->bytes, true)) return;
+    if (!L->rest || !two_steps_pay(&L->desc, L->bytes, true)) return;
     const bgk_sweep_params& p = L->p;
     const long long nodes = (long long)(p.imax - p.imin + 3) * (p.jmax - p.jmin + 3) * (p.kmax - p.kmin + 3);
     void* buf = nullptr;
@@ -370,10 +380,12 @@ void bgk_lattice_desc_init(bgk_lattice_desc* d, int kind, int bcase, int l, int 
     d->scale = 1.0f;
 }
 
-size_t bgk_lattice_device_bytes(const bgk_lattice_desc* d) {
+size_t bgk_lattice_least_bytes(const bgk_lattice_desc* d) {
     const Geometry g = geometry(d);
     return (size_t)g.plane * nplanes(d) * elem_bytes(d->kind);
 }
+
+size_t bgk_lattice_device_bytes(const bgk_lattice_desc* d) { return bgk_lattice_least_bytes(d) + rest_bytes(d); }
 
 int bgk_lattice_create(const bgk_lattice_desc* d, bgk_lattice** out) {
     if (!d || !out) return set_error(BGK_ERR_ARG, "null argument");
@@ -394,13 +406,11 @@ int bgk_lattice_create(const bgk_lattice_desc* d, bgk_lattice** out) {
     L->p.scale = d->scale;
     L->p.fast = d->fast;
     if (int e = validate(&L->p)) { delete L; return e; }
-    L->bytes = bgk_lattice_device_bytes(d);
-    // a lattice whose steps run four at a time has one array more, the rest
-    // population's second one (two-step sweep, 32-bit byte offsets), in the
-    // same block of memory; without room for it, it takes single steps
-    const size_t array = (size_t)L->plane * L->es;
-    const bool fours = d->pattern == BGK_PATTERN_AB && two_steps_pay(L->p, L->bytes, false) && array < (1ULL << 32);
-    int rc = fours ? dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes + array, true, "lattice") : BGK_ERR_NOMEM;
+    L->bytes = bgk_lattice_least_bytes(d);
+    // the rest population's second array in the same block of memory; without
+    // room for it, the lattice takes single steps
+    const size_t rest = rest_bytes(d);
+    int rc = rest ? dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes + rest, true, "lattice") : BGK_ERR_NOMEM;
     if (rc == BGK_OK) L->rest = L->base + L->bytes + (size_t)(L->shift + L->origin) * L->es;
     else rc = dev_alloc(reinterpret_cast<void**>(&L->base), L->bytes, true, "lattice");
     if (rc) {

@@ -103,7 +103,10 @@ def extents(req: Request):
     return s, s, s, {"ldc": "driven", "tgv": "periodic"}[req.case]
 
 
-def lattice_bytes(req: Request) -> int:
+def _bytes(req: Request):
+    """(bytes a request's lattice takes, bytes it cannot do without): its arrays,
+    and in the first the table of solid links of a sphere's box grown by one
+    node where its steps run two per launch."""
     from .lattice import lib
     from ._lattice_abi import LatticeDesc
     import ctypes
@@ -112,7 +115,14 @@ def lattice_bytes(req: Request) -> int:
     kind = {"f32": 1, "f16": 2}[req.kind]
     lib().bgk_lattice_desc_init(ctypes.byref(d), kind, {"driven": 0, "periodic": 1, "channel": 2,
                                                        "inflow": 3}[bcase], l, m, n, 1.0 / req.tau)
-    return int(lib().bgk_lattice_device_bytes(ctypes.byref(d)))
+    full, least = (int(f(ctypes.byref(d))) for f in (lib().bgk_lattice_device_bytes, lib().bgk_lattice_least_bytes))
+    if req.case == "sphere" and full > least:
+        full += 4 * (int(max(4.0, req.side / 6.0)) + 3) ** 3
+    return full, least
+
+
+def lattice_bytes(req: Request) -> int:
+    return _bytes(req)[0]
 
 
 class _Active:
@@ -122,7 +132,7 @@ class _Active:
         self.lat = CS.make_lattice(self.case, fast=req.fast)
         self.remaining = req.steps
         self.t_admit = t_admit
-        self.bytes = self.lat.device_bytes
+        self.bytes = lattice_bytes(req)
         self.nodes = self.case["l"] * self.case["m"] * self.case["n"]
 
     def result(self) -> dict:
@@ -169,6 +179,14 @@ class Server:
                 break
         return sel
 
+    def _need(self, req: Request) -> int:
+        """Bytes of a request's lattice.  One that the budget holds only without
+        what two steps per launch work with (a 38th of it) is admitted, alone."""
+        need, least = _bytes(req)
+        if least > self.budget:
+            raise RuntimeError(f"request {req.rid} needs {least} bytes, more than the budget")
+        return need
+
     def run(self, trace, mode: str = "continuous", keep_states: bool = False):
         """Serve the trace; returns (per-request records, summary)."""
         if mode not in ("continuous", "shared", "fifo", "plain"):
@@ -191,10 +209,8 @@ class Server:
             nonlocal used, t_admit
             ta = time.perf_counter()
             while pending and pending[0].arrival <= now:
-                need = lattice_bytes(pending[0])
-                if need > self.budget:
-                    raise RuntimeError(f"request {pending[0].rid} needs {need} bytes, more than the budget")
-                if (one_at_a_time and active) or used + need > self.budget:
+                need = self._need(pending[0])
+                if active and (one_at_a_time or used + need > self.budget):
                     break
                 a = _Active(pending.pop(0), now)
                 active.append(a)
@@ -307,10 +323,8 @@ class Server:
             nonlocal used, t_admit, next_stream
             ta = time.perf_counter()
             while pending and pending[0].arrival <= now:
-                need = lattice_bytes(pending[0])
-                if need > self.budget:
-                    raise RuntimeError(f"request {pending[0].rid} needs {need} bytes, more than the budget")
-                if used + need > self.budget:
+                need = self._need(pending[0])
+                if active and used + need > self.budget:
                     break
                 a = _Active(pending.pop(0), now)
                 a.stream = self.streams[next_stream % nstreams]

@@ -44,12 +44,15 @@ typedef struct bgk_lattice_desc {
 /* Defaults: AB pattern, no force, lid 0, inflow 0, scale 1, fast 0. */
 void bgk_lattice_desc_init(bgk_lattice_desc* d, int kind, int bcase, int l, int m, int n, double omega);
 
-/* Device bytes a lattice with this description needs (admission control).  An
-   AB lattice of a 4- or 8-byte kind takes one more population array (1/37)
-   where the device has room for it, and with an obstacle 4 bytes per node of
-   the obstacle's box: what its two-step launches work with.  Without them it
-   takes single steps. */
+/* Device bytes of the arrays that a lattice with this description takes
+   (admission control).  An AB lattice whose steps run two per launch takes one
+   more population array (38 instead of 37), and with an obstacle 4 bytes per
+   node of the obstacle's box and its neighbours, which the figure does not
+   hold, as it does not hold the obstacle's mask.  Where the device has no room
+   for these, it is created all the same and takes single steps:
+   bgk_lattice_least_bytes is what it cannot do without. */
 size_t bgk_lattice_device_bytes(const bgk_lattice_desc* d);
+size_t bgk_lattice_least_bytes(const bgk_lattice_desc* d);
 
 /* Allocate the lattice on the current device.  Lattices, batches and their
    masks and workspaces come from one stream-ordered memory pool per device;

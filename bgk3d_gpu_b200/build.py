@@ -29,7 +29,8 @@ NVCC_FLAGS = ARCH + [
 ]
 
 LIB_SOURCES = ["bgk_api.cu", "lattice.cu", "lattice_io.cu", "diag.cu", "batch.cu", "noalloc.cu", "devmem.cu"] + [
-    f"inst_{kind}_{group}.cu" for kind in ("f64", "f32", "f16", "bf16", "f32f64") for group in ("ab", "t2", "aa", "batch", "misc")]
+    f"inst_{kind}_{group}.cu" for kind in ("f64", "f32", "f16", "bf16", "f32f64") for group in ("ab", "aa", "batch", "misc")] + [
+    f"inst_{kind}_t2.cu" for kind in ("f64", "f32", "f32f64")]
 LIB = "libbgk3d_b200.so"
 DROPIN_SP = "libbgk3d_dropin_sp.so"
 DROPIN_DP = "libbgk3d_dropin_dp.so"
@@ -75,7 +76,7 @@ def build(force: bool = False, verbose: bool = False) -> dict:
     for src in LIB_SOURCES:
         srcp = os.path.join(CSRC, src)
         if not os.path.exists(srcp):
-            continue
+            raise RuntimeError(f"source {srcp} is missing")
         obj = os.path.join(PKG, "_build", src.replace(".cu", ".o"))
         objs.append(obj)
         if force or _stale(obj, deps):

@@ -309,11 +309,12 @@ def fp16_accuracy(steps: int = 2000):
     return out
 
 
-def step_launches(start, steps, pattern):
-    """Kernel launches of lat.step(steps) from step count start: the AB lattice
-    takes four steps as two launches (two steps per pass over memory), a long
-    run from an odd count one single step first; AA steps are one launch each."""
-    if pattern != "ab":
+def step_launches(start, steps, two_steps):
+    """Kernel launches of lat.step(steps) from step count start: a lattice that
+    takes two steps per launch (Lattice.uses_two_steps) takes four steps as two
+    launches, and a long run from an odd count one single step first; the others
+    launch once per step."""
+    if not two_steps:
         return steps
     first = 1 if steps >= 32 and start % 2 else 0
     return first + 2 * ((steps - first) // 4) + (steps - first) % 4
@@ -402,9 +403,9 @@ def run_ours(args):
     time.sleep(0.3)
     from bgk3d_gpu_b200.replicas import job_throughput
     nodes = L_ * M_ * N_
-    region_ms, launched = [], 0
+    region_ms, launched, two_steps = [], 0, lat.uses_two_steps
     for _ in range(repeats):
-        launched += step_launches(lat.steps, args.steps, args.pattern)
+        launched += step_launches(lat.steps, args.steps, two_steps)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         torch.cuda.synchronize()
         _barrier(ws)
@@ -465,8 +466,7 @@ def run_ours(args):
                      "frac": achieved / peak, "peak_source": peak_src,
                      "traffic": None,
                      "traffic_note": "no counter is read in this run: DRAM read + write per launch from ncu "
-                                     "are in profiles/" + ("sweep_t2_f32.md" if args.pattern == "ab" else
-                                                           "kernel_sweep_256.md"),
+                                     "are in profiles/",
                      "algorithmic_bytes_per_launch": B_ALG_F32 * nodes,
                      "b_alg_per_lup": B_ALG_F32 * launches / args.steps,
                      "note": "two steps per pass: bound by instruction issue, not by HBM" if launches < args.steps else "",

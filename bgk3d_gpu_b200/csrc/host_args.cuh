@@ -146,7 +146,15 @@ inline int row_lanes(int pairs, bool fifth) {
     }
     return best;
 }
-// Geometry of the pair kernels; returns the warps of one step.  The forms for
+// Multiprocessors of the current device.
+inline int sm_count() {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
+// Geometry of the pair kernels on a device of nsm multiprocessors; returns the warps of one step.  The forms for
 // cut rows of three kinds of launch are much slower warp for warp than those for
 // whole-warp segments.  The driven cavity's odd AA step (waves) and launches with
 // an inflow face or an obstacle cut only where whole warps come to more than run
@@ -154,11 +162,11 @@ inline int row_lanes(int pairs, bool fifth) {
 // 10.52), the latter two also for a larger share only (FP16 fast inflow 144x96x96,
 // 72 of 96 lanes, 40.6 -> 43.7 GLUPS; 200x140x140, 104 of 128, 47.1 -> 45.8).
 template <class S, class C>
-long long pair_geometry(SweepArgs<S, C>& A, bool waves, bool obs) {
+long long pair_geometry(SweepArgs<S, C>& A, bool waves, bool obs, int nsm) {
     const bool slow = obs || A.bcase == BC_INFLOW;
     const int pairs = A.l / 2;
     const long long rows = (long long)A.m * A.n;
-    const long long resident = 148LL * kPairBlocks * (kPairThreads / 32);
+    const long long resident = (long long)nsm * kPairBlocks * (kPairThreads / 32);
     A.gs = (waves || slow) && rows * ((pairs + 31) / 32) <= resident ? 5 : row_lanes(pairs, slow);
     A.lmask = (1 << A.gs) - 1;
     A.nseg = (pairs + A.lmask) >> A.gs;

@@ -182,7 +182,7 @@ int launch_sweep(const bgk_sweep_params* p, void* const* a, void* const* b, doub
         if (g_pair_kernels && mom == nullptr && nelem < (1LL << 31) && pairs_aligned<S>(p, a, b)) {
             // adjacent node pairs
             SweepArgs<S, C> A2 = A;
-            const long long w2 = pair_geometry(A2, false, obs);
+            const long long w2 = pair_geometry(A2, false, obs, sm_count());
             constexpr int wpb = kPairThreads / 32;
             const unsigned nb2 = (unsigned)((w2 + wpb - 1) / wpb);
             switch (p->bcase) {
@@ -252,9 +252,8 @@ template <class S, class C, int BC, int CM, bool OBS>
 int launch_t2_variant(const SweepArgs<S, C>& A, const uint32_t* links, int* err, cudaStream_t st) {
     typedef T2Lay<S, C, BC, OBS> R;
     auto kern = sweep_t2_kernel<S, C, BC, CM, OBS>;
-    int dev = 0, nsm = 0;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     static std::atomic<unsigned long long> ready{0};   // devices on which the kernel's shared-memory limit is raised
     if (!(ready.load(std::memory_order_acquire) >> (dev & 63) & 1)) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, R::BYTES);
@@ -266,7 +265,7 @@ int launch_t2_variant(const SweepArgs<S, C>& A, const uint32_t* links, int* err,
     Q.links = links;
     Q.err = err;
     for (int d = 0; d < 19; ++d) Q.src[d] = A.a[d] - (cx_of(d) + cy_of(d) * A.nx + cz_of(d) * A.nxy);
-    Q.g = t2_tiles(A.l, A.m, A.n, R::TX, R::H, nsm * T2Cfg<C>::BLOCKS, t2_uneven<BC>(OBS),
+    Q.g = t2_tiles(A.l, A.m, A.n, R::TX, R::H, sm_count() * T2Cfg<C>::BLOCKS, t2_uneven<BC>(OBS),
                      sizeof(C) == 4 ? 0.5 : 0.85);
     const long long units = (long long)Q.g.ntx * Q.g.nty * ((A.n + Q.g.zc - 1) / Q.g.zc);
     kern<<<(unsigned)units, R::THREADS, R::BYTES, st>>>(Q);
@@ -548,7 +547,7 @@ int launch_aa(const bgk_sweep_params* p, void* const* slots, bool odd, double* m
             constexpr int wpb = kPairThreads / 32;
             const bool obs = A.obs != nullptr, inflow = p->bcase == BC_INFLOW;
             const unsigned nb2 =
-                (unsigned)((pair_geometry(A2, odd && p->bcase == BC_DRIVEN, obs) + wpb - 1) / wpb);
+                (unsigned)((pair_geometry(A2, odd && p->bcase == BC_DRIVEN, obs, sm_count()) + wpb - 1) / wpb);
             if (!odd) {
                 if (inflow) {
                     if (obs) launch_aa_even_pair<S, C, true, true>(A2, cm, nb2, st);

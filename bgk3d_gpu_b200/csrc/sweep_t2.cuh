@@ -8,12 +8,12 @@
 // first step into a ring of planes in shared memory, and the tile one plane
 // behind by the second step from the ring into b.  Per two updates a node is
 // read once and written once, plus the rims, which neighbouring blocks read at
-// about the same time (DRAM reads 1.07x the algorithmic bytes at 256x256x128).
+// about the same time (DRAM reads 1.03x the algorithmic bytes at 256x256x128).
 // The state in between is rounded to storage precision, so the results are bit
 // for bit those of two one-step launches, every face and obstacle included.
 //
-// What bounds it now is instruction issue (FP32 256^3: 600 thread-instructions
-// per warp and plane for the two collisions, 76 % of the issue slots, DRAM at
+// What bounds it now is instruction issue (FP32 256x256x128: 486
+// thread-instructions per update, rims included, 75 % of the issue slots, DRAM at
 // half its rate).  What the layout rests on, each measured at 256^3:
 //  * a thread reads the 19 values of the next plane straight into registers
 //    before its second step, so that the loads are in flight while it works;
@@ -25,8 +25,8 @@
 //    back).  Most of the 256 KB stays L1, whose size bounds the loads in
 //    flight: a ring over all of shared memory ran at 27 GLUPS;
 //  * two blocks per SM, so that one works while the other waits: 57 against 51
-//    for one block of twice the size.  FP32 11 warps (88 registers) 59.0, 13
-//    warps 57.4, 16 warps (64 registers) 52.6; FP64 6 warps (168 registers)
+//    for one block of twice the size.  FP32 11 warps (76-80 registers) 59.0, 13
+//    warps 57.4, 16 warps (at most 64) 52.6; FP64 6 warps (146-160 registers)
 //    31.0, 5 warps x 3 blocks 30.4, 8 warps 28.0;
 //  * split barriers: a warp arrives when its plane is stored or read and waits
 //    only before it needs the others' (59.0 -> 59.6 FP32, 48.3 -> 56.6 FP32

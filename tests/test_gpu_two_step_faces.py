@@ -2,6 +2,8 @@
 where the rims of the tiles that wrap around a periodic axis have links into
 solid nodes, and runs that start at an odd step count: the same bits in every
 array cell as single steps (which take the one-step sweep)."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -29,6 +31,11 @@ def solids_at(shape, place, seed=4):
     return obs
 
 
+@functools.lru_cache(maxsize=2)
+def state(shape, kind):
+    return random_state(*shape, kind, seed=shape[0] + kind)
+
+
 def run(shape, kind, case, calls, obs=None, fast=False):
     from bgk3d_gpu_b200.lattice import Lattice
     from test_gpu_lattice import lattice_kwargs
@@ -36,7 +43,7 @@ def run(shape, kind, case, calls, obs=None, fast=False):
     if obs is not None:
         lat.set_obstacle(obs)
     assert lat.uses_two_steps or kind == 4
-    lat.upload(random_state(*shape, kind, seed=shape[0] + kind))
+    lat.upload(state(shape, kind))
     for c in calls:
         lat.step(c)
     out = lat.download()
@@ -45,7 +52,8 @@ def run(shape, kind, case, calls, obs=None, fast=False):
 
 
 def differing(a, b):
-    return int((a.view(np.uint8) != b.view(np.uint8)).sum())
+    a, b = (x.view(np.uint64 if x.itemsize == 8 else np.uint32) for x in (a, b))
+    return int((a != b).sum())
 
 
 @pytest.mark.parametrize("case", ["periodic", "channel", "inflow", "driven"])
@@ -93,3 +101,9 @@ def test_runs_that_start_at_an_odd_step_count(case, calls):
     shape = SHAPES[case]
     obs = solids_at(shape, (0, 0, 0)) if case == "inflow" else None
     assert differing(run(shape, 1, case, calls, obs), run(shape, 1, case, (1,) * sum(calls), obs)) == 0
+
+
+@pytest.mark.parametrize("case", ["periodic", "channel", "inflow", "driven"])
+@pytest.mark.parametrize("shape", [(1000, 900, 1), (900, 1, 1100), (1, 200, 170), (2, 170, 200), (640, 900, 2), (3, 190, 180)])
+def test_lattices_of_one_to_three_nodes_along_an_axis(case, shape):
+    assert differing(run(shape, 1, case, (4, 5), None), run(shape, 1, case, (1,) * 9, None)) == 0

@@ -119,3 +119,31 @@ def test_lines_of_the_dispatch(kind, case, shape, sphere, two):
         c.close()
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("kind,case,shape,part,fill,two", [
+    (1, "driven", (128, 100, 90), 1.0, 0.3, True),       # porous: fluid nodes all over the box
+    (1, "driven", (128, 100, 90), 0.4, 0.3, False),      # a body: below the line for obstacles
+    (0, "periodic", (100, 70, 70), 0.8, 0.2, True), (0, "periodic", (128, 100, 90), 0.8, 1.0, False),   # a block
+    (0, "inflow", (128, 90, 90), 0.8, 0.3, True), (4, "channel", (128, 100, 90), 1.0, 0.3, False),
+])
+def test_obstacles_by_their_share_of_the_lattice(kind, case, shape, part, fill, two):
+    """Solid nodes at random in a part of every extent: the route, and the same fluid state as by single steps."""
+    l, m, n = shape
+    rng = np.random.default_rng(2)
+    obs = np.zeros((n, m, l), np.int32)
+    at = tuple(slice(1 + (e - 2 - int((e - 2) * part)) // 2, 1 + (e - 2 - int((e - 2) * part)) // 2 + int((e - 2) * part)) for e in (n, m, l))
+    obs[at] = rng.random(obs[at].shape) < fill
+    st0 = random_state(*shape, kind, seed=13)
+    lats = [lattice(shape, case, kind, state=st0) for _ in range(2)]
+    for lat in lats:
+        lat.set_obstacle(obs)
+        assert lat.uses_two_steps == two
+    lats[0].step(6)
+    for _ in range(6):
+        lats[1].step(1)
+    assert status(lats[0]) == 0
+    a, b = (lat.download().view(np.uint8) for lat in lats)
+    assert np.array_equal(a, b)
+    for lat in lats:
+        lat.close()

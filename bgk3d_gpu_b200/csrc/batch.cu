@@ -226,8 +226,9 @@ int build_groups(bgk_batch* B) {
     if (B->chunk <= 0) return BGK_OK;
     std::vector<int> alone;
     for (size_t i = 0; i < B->lats.size(); ++i) {
-        B->in_fours[i] = bgk_lat::steps_in_fours(B->lats[i], &B->made[i]) ? 1 : 0;
-        if (B->in_fours[i] || is_solo(B, (int)i)) alone.push_back((int)i);
+        const bool solo = is_solo(B, (int)i);
+        B->in_fours[i] = (solo ? bgk_lat::steps_in_fours_alone : bgk_lat::steps_in_fours)(B->lats[i], &B->made[i]) ? 1 : 0;
+        if (B->in_fours[i] || solo) alone.push_back((int)i);
     }
     for (const bgk_batch::Group& g : B->groups) {
         bgk_batch::Group o = g;

@@ -107,15 +107,19 @@ int one_step(bgk_lattice* L, cudaStream_t st, double* mom = nullptr, double* mom
 }
 
 // Where a lattice's steps run four at a time, as two launches of two steps each
-// (sweep_t2.cuh): where that was the faster way at 6279 shapes of 15 MB to 4 GB
-// (l 7 to 256, m : n from 1 : 4 to 4 : 1, 32 to 64 steps through the captured
-// graph, with and without a sphere).  Two lines, both in bytes of all arrays:
-//  * the allocation, padding included, has to outgrow the 126 MB L2, from which
-//    the one-step sweep runs below it: two_step_line;
-//  * so have the 128-byte lines that hold nodes, or MiB as follows.  Below, the
-//    one-step sweep still finds part of its state in L2, and the two-step sweep
-//    has few blocks, whose slowest ends the launch: those at a wall or at an
-//    obstacle.  Two steps per pass ran at 0.74-0.95 of one for FP64 periodic and
+// (sweep_t2.cuh).  Two lines, both in MiB of all arrays:
+//  * two_step_line: the allocation, padding included, has to outgrow the 126 MB
+//    L2, from which the one-step sweep runs below it.  In a batch that is all:
+//    its groups' launches are slower than a lattice's own, and its branches fill
+//    the ends of each other's launches (2 to 16 members of sides 72 to 160, two
+//    steps per pass against groups: FP32 1.03-1.64, with a sphere 1.02-1.46; FP64
+//    1.05-1.73 and 1.0-1.37; FP32/FP64 mixed 1.0-1.35);
+//  * two_steps_pay: a lattice that steps alone goes by the 128-byte lines that
+//    hold nodes as well, by what was the faster way at 6279 shapes of 15 MB to 4 GB
+//    (l 7 to 256, m : n from 1 : 4 to 4 : 1, 32 to 64 steps through the captured
+//    graph, with and without a sphere).  Below, the one-step sweep still finds
+//    part of its state in L2, and the two-step sweep has few blocks, whose slowest
+//    ends the launch: those at a wall or at an obstacle.  Two steps per pass ran at 0.74-0.95 of one for FP64 periodic and
 //    driven rows of 17 to 32 nodes below 100 MiB, with a sphere at 0.73-0.98
 //    (FP32 driven, 90-300 MiB) and 0.61-1.0 (FP64 driven, to 300 MiB); from the
 //    lines below it gains.
@@ -144,25 +148,23 @@ size_t two_step_node_line(int kind, int bcase, int l, bool obstacle) {
     if (obstacle) return kNever;
     return idle ? 60 : (bcase == BC_INFLOW ? 1000 : kNever);
 }
-// bytes: the arrays of the lattice d describes.
-bool two_steps_pay(const bgk_lattice_desc* d, size_t bytes, bool obstacle) {
-    if (d->kind != K_F64 && d->kind != K_F32 && d->kind != K_F32_F64) return false;
-    if (d->bcase < BC_DRIVEN || d->bcase > BC_INFLOW || d->pattern != BGK_PATTERN_AB) return false;
+bool two_steps_pay(const bgk_lattice_desc* d, bool obstacle) {
     const size_t row = ((size_t)d->l * elem_bytes(d->kind) + 127) / 128 * 128;
-    return (bytes >> 20) >= two_step_line(d->bcase) &&
-           (37 * row * (size_t)d->m * (size_t)d->n >> 20) >= two_step_node_line(d->kind, d->bcase, d->l, obstacle);
+    return (37 * row * (size_t)d->m * (size_t)d->n >> 20) >= two_step_node_line(d->kind, d->bcase, d->l, obstacle);
 }
 
 // Bytes of one more array, the rest population's second one, which a lattice
-// whose steps run four at a time has behind its arrays (two-step sweep, 32-bit
-// byte offsets); 0 for the others.
+// whose steps may run four at a time, alone or in a batch, has behind its arrays
+// (two-step sweep, 32-bit byte offsets); 0 for the others.
 size_t rest_bytes(const bgk_lattice_desc* d) {
+    if (d->kind != K_F64 && d->kind != K_F32 && d->kind != K_F32_F64) return 0;
+    if (d->bcase < BC_DRIVEN || d->bcase > BC_INFLOW || d->pattern != BGK_PATTERN_AB) return 0;
     const size_t array = (size_t)geometry(d).plane * elem_bytes(d->kind);
-    return two_steps_pay(d, array * nplanes(d), false) && array < (1ULL << 32) ? array : 0;
+    return (37 * array >> 20) >= two_step_line(d->bcase) && array < (1ULL << 32) ? array : 0;
 }
 
-// Whether an open lattice that takes two steps per launch does so with its
-// obstacle of `solid` nodes.  The one-step sweep takes longest where fluid nodes
+// Whether a lattice that steps alone takes two steps per launch with its obstacle
+// of L->solid nodes.  The one-step sweep takes longest where fluid nodes
 // lie near solid ones (19 mask entries each) and least inside a solid, which the
 // two-step sweep computes and does not store.  Two steps per pass against one
 // (80-2000 MiB):
@@ -172,20 +174,23 @@ size_t rest_bytes(const bgk_lattice_desc* d) {
 //  * a quarter of the lattice solid and no such share of fluid nodes (blocks): FP32
 //    0.85-1.15, FP64 0.79-1.12;
 //  * otherwise (bodies in the flow) the lines for obstacles.
-bool two_steps_pay_with(const bgk_lattice* L, long long solid) {
+bool two_steps_pay_with_obstacle(const bgk_lattice* L) {
     const bgk_sweep_params& p = L->p;
+    const long long solid = L->solid;
     const long long nodes = (long long)p.l * p.m * p.n;
     const long long box = (long long)(p.imax - p.imin + 1) * (p.jmax - p.jmin + 1) * (p.kmax - p.kmin + 1);
-    if (p.kind != K_F32_F64 && 12 * (box - solid) >= nodes) return true;
-    return 4 * solid < nodes && two_steps_pay(&L->desc, L->bytes, true);
+    if (p.kind != K_F32_F64 && 12 * (box - solid) >= nodes) return two_steps_pay(&L->desc, false);
+    return 4 * solid < nodes && two_steps_pay(&L->desc, true);
 }
 
 // The table of solid links the two-step sweep reads (t2_links_kernel), made
-// for the lattice's current obstacle; without it (no memory left, or two steps
-// per pass do not pay with the obstacle) the lattice takes single steps.
+// for the lattice's current obstacle; without it (no memory left, or a mixed
+// FP32/FP64 lattice but inflow, which runs at 0.79-1.03 of a batch's groups with
+// it) the lattice takes single steps.
 void make_links(bgk_lattice* L, long long solid) {
-    if (!L->rest || !two_steps_pay_with(L, solid)) return;
     const bgk_sweep_params& p = L->p;
+    L->solid = solid;
+    if (!L->rest || (p.kind == K_F32_F64 && p.bcase != BC_INFLOW)) return;
     const long long nodes = (long long)(p.imax - p.imin + 3) * (p.jmax - p.jmin + 3) * (p.kmax - p.kmin + 3);
     void* buf = nullptr;
     if (dev_alloc(&buf, (size_t)nodes * sizeof(uint32_t), false, "solid links") != BGK_OK) return;
@@ -356,6 +361,11 @@ bool steps_in_fours(const bgk_lattice* L, const bgk_sweep_params* p) {
     return L->rest && (!has_obs || L->links) && !p->zhalo;
 }
 
+bool steps_in_fours_alone(const bgk_lattice* L, const bgk_sweep_params* p) {
+    if (!steps_in_fours(L, p)) return false;
+    return L->links ? two_steps_pay_with_obstacle(L) : two_steps_pay(&L->desc, false);
+}
+
 int four_steps(const bgk_lattice* L, const bgk_sweep_params* p, void* const* a, void* const* b, bool outflow_fresh,
                cudaStream_t st) {
     void* t[19];
@@ -473,7 +483,7 @@ int bgk_lattice_uses_tma(const bgk_lattice* L) {
 }
 
 int bgk_lattice_uses_two_steps(const bgk_lattice* L) {
-    return (L && bgk_lat::steps_in_fours(L, &L->p) && !(L->tma_ok && g_tma_kernels)) ? 1 : 0;
+    return (L && bgk_lat::steps_in_fours_alone(L, &L->p) && !(L->tma_ok && g_tma_kernels)) ? 1 : 0;
 }
 
 int bgk_lattice_set_zhalo(bgk_lattice* L, int flags) {

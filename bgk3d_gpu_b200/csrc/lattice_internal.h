@@ -21,6 +21,7 @@ struct bgk_lattice {
     void* rest = nullptr;        // AB, large: a second array of population 19 at element (0,0,0) (two-step sweep), or null
     uint32_t* links = nullptr;   // with an obstacle: its table of solid links (two-step sweep), or null
     int32_t* obs_dev = nullptr;
+    long long solid = 0;         // its solid nodes (a sphere's: from its volume)
     long long obs_version = 0;   // raised whenever the obstacle's mask and table are replaced
     long long steps = 0;
     double* ws = nullptr;
@@ -43,10 +44,12 @@ struct bgk_lattice {
 // Shared by the lattice's host-transfer paths (lattice.cu, lattice_io.cu) and
 // the batched stepper.
 namespace bgk_lat {
-// True when the lattice's steps with the parameters p run four at a time (AB,
-// arrays that outgrow L2, rest population's second array and obstacle table
-// in place).
+// True when the lattice's steps with the parameters p can run four at a time
+// (AB, arrays that outgrow L2, rest population's second array and obstacle table
+// in place), as those of a batch's group members do; _alone: where that is also
+// faster than its own one-step launches.
 bool steps_in_fours(const bgk_lattice* L, const bgk_sweep_params* p);
+bool steps_in_fours_alone(const bgk_lattice* L, const bgk_sweep_params* p);
 // Four steps with the parameters p as two two-step launches a -> b -> a.  The arrays end as four
 // single steps leave them: a holds the state, and neither the halo nor the
 // solid nodes of either set are written (an inflow lattice's outflow plane

@@ -290,10 +290,10 @@ int launch_t2_cm(const SweepArgs<S, C>& A, int cm, const uint32_t* links, int* e
 template <class S, class C, int BC>
 int launch_t2_bc(const SweepArgs<S, C>& A, const uint32_t* links, int* err, cudaStream_t st) {
     const int cm = coll_mode(A);
-    if constexpr (sizeof(S) == sizeof(C)) {
+    if constexpr (sizeof(S) == sizeof(C) || BC == BC_INFLOW) {
         if (A.obs) return launch_t2_cm<S, C, BC, true>(A, cm, links, err, st);
     } else {
-        if (A.obs) return set_error(BGK_ERR_UNSUPPORTED, "two-step sweep: no obstacles in mixed precision");
+        if (A.obs) return set_error(BGK_ERR_UNSUPPORTED, "two-step sweep: mixed precision with an obstacle: inflow only");
     }
     return launch_t2_cm<S, C, BC, false>(A, cm, nullptr, err, st);
 }

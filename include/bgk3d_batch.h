@@ -62,8 +62,9 @@ int bgk_batch_set_solo(bgk_batch* batch, long long min_nodes);
 long long bgk_batch_get_solo(const bgk_batch* batch);
 int bgk_batch_groups(const bgk_batch* batch);
 
-/* Members whose steps run four at a time, as two launches of two steps each
-   (bgk_lattice_uses_two_steps), in the batch's present form. */
+/* Members whose steps run four at a time, as two launches of two steps each, in
+   the batch's present form: smaller ones too than those that do so alone
+   (bgk_lattice_uses_two_steps), since a group's launch is the slower one. */
 int bgk_batch_two_step_members(const bgk_batch* batch);
 
 /* Tile queue parameters: tiles taken per queue access (1..16) and resident

@@ -45,8 +45,8 @@ typedef struct bgk_lattice_desc {
 void bgk_lattice_desc_init(bgk_lattice_desc* d, int kind, int bcase, int l, int m, int n, double omega);
 
 /* Device bytes of the arrays that a lattice with this description takes
-   (admission control).  An AB lattice whose steps run two per launch takes one
-   more population array (38 instead of 37), and with an obstacle 4 bytes per
+   (admission control).  An AB lattice whose steps may run two per launch, alone
+   or in a batch, takes one more population array (38 instead of 37), and with an obstacle 4 bytes per
    node of the obstacle's box and its neighbours, which the figure does not
    hold, as it does not hold the obstacle's mask.  Where the device has no room
    for these, it is created all the same and takes single steps:
@@ -140,7 +140,7 @@ long long bgk_io_set_subrecord_limit(long long bytes);
 /* Advance nsteps time steps (boundaries + stream + collide), stream-ordered.
    Runs of 32 or more steps replay a captured 16-step CUDA graph (captured on
    the first such run unless bgk_lattice_prepare captured it before).  AB
-   lattices of the 4- and 8-byte kinds whose arrays outgrow the L2 cache take
+   lattices of the 4- and 8-byte kinds take, where that is faster (large ones),
    four steps at a time as two launches of two steps each; the state outside
    solid nodes is bit for bit that of single steps. */
 int bgk_lattice_step(bgk_lattice* lat, int nsteps, void* stream);

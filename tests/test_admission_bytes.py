@@ -21,8 +21,7 @@ def figures(d):
 
 @pytest.mark.parametrize("kind,bcase,shape,pattern,arrays", [
     (1, 1, (256, 256, 256), 0, 38), (0, 0, (128, 128, 128), 0, 38), (1, 3, (512, 256, 256), 0, 38),
-    (4, 1, (40, 150, 110), 0, 38),
-    (4, 1, (256, 256, 256), 0, 37), (1, 1, (32, 32, 32), 0, 37), (2, 1, (256, 256, 256), 0, 37), (1, 1, (256, 256, 256), 1, 19),
+    (4, 1, (40, 150, 110), 0, 38), (4, 1, (256, 256, 256), 0, 38), (1, 1, (32, 32, 32), 0, 37), (2, 1, (256, 256, 256), 0, 37), (1, 1, (256, 256, 256), 1, 19),
     (1, 1, (1200, 1000, 900), 0, 37),            # an array of 4 GB or more takes single steps
 ])
 def test_arrays_counted(kind, bcase, shape, pattern, arrays):

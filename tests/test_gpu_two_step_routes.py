@@ -147,3 +147,32 @@ def test_obstacles_by_their_share_of_the_lattice(kind, case, shape, part, fill, 
     assert np.array_equal(a, b)
     for lat in lats:
         lat.close()
+
+
+@pytest.mark.parametrize("kind,sphere", [(0, False), (1, False), (4, False), (0, True), (1, True), (4, True)])
+def test_group_members_take_two_steps_earlier_than_lattices_alone(kind, sphere):
+    """Members between the two lines: in rounds of four in a batch's groups, by
+    single steps alone and as solo members; the same states, mixed precision
+    with an obstacle included (inflow only)."""
+    from bgk3d_gpu_b200.lattice import Batch
+    specs = {0: [("driven", (72, 72, 72)), ("periodic", (20, 95, 95)), ("channel", (20, 95, 95))],
+             1: [("driven", (96, 90, 90)), ("periodic", (20, 160, 110)), ("inflow", (128, 120, 110))],
+             4: [("driven", (128, 90, 90)), ("periodic", (128, 80, 80)), ("inflow", (128, 120, 110))]}[kind]
+    st = [random_state(*shape, kind, seed=17 + q) for q, (_, shape) in enumerate(specs)]
+    alone, lats = ([lattice(shape, case, kind, sphere, s) for (case, shape), s in zip(specs, st)] for _ in range(2))
+    batch = Batch(lats)
+    members = batch.two_step_members
+    assert members == (1 if kind == 4 and sphere else 3)
+    assert sum(lat.uses_two_steps for lat in lats) < members
+    batch.step(21)
+    batch.set_solo(1)
+    assert batch.two_step_members == sum(lat.uses_two_steps for lat in lats)
+    batch.step(5)
+    for a, b in zip(alone, lats):
+        for _ in range(26):
+            a.step(1)
+        assert status(b) == 0
+        assert np.array_equal(a.download().view(np.uint8), b.download().view(np.uint8))
+    batch.close()
+    for lat in alone + lats:
+        lat.close()

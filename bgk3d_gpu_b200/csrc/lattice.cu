@@ -115,42 +115,50 @@ int one_step(bgk_lattice* L, cudaStream_t st, double* mom = nullptr, double* mom
 //    steps per pass against groups: FP32 1.03-1.64, with a sphere 1.02-1.46; FP64
 //    1.05-1.73 and 1.0-1.37; FP32/FP64 mixed 1.0-1.35);
 //  * two_steps_pay: a lattice that steps alone goes by the 128-byte lines that
-//    hold nodes as well, by what was the faster way at 6279 shapes of 15 MB to 4 GB
-//    (l 7 to 256, m : n from 1 : 4 to 4 : 1, 32 to 64 steps through the captured
-//    graph, with and without a sphere).  Below, the one-step sweep still finds
-//    part of its state in L2, and the two-step sweep has few blocks, whose slowest
-//    ends the launch: those at a wall or at an obstacle.  Two steps per pass ran at 0.74-0.95 of one for FP64 periodic and
-//    driven rows of 17 to 32 nodes below 100 MiB, with a sphere at 0.73-0.98
-//    (FP32 driven, 90-300 MiB) and 0.61-1.0 (FP64 driven, to 300 MiB); from the
-//    lines below it gains.
-// The one-step sweep's warps take 32 nodes of a row, the two-step tiles of FP64
-// arithmetic 16: rows that leave a quarter or more of the former's lanes without
-// a node that the latter's have (l to 16, 33 to 48) gain earlier.  FP32 storage
-// with FP64 arithmetic moves half of FP64's bytes for its instructions, so the
-// rims' second computation costs more than a pass saves (0.66-1.08 of one step
-// per pass, with a sphere 0.54-1.0 at most shapes) but for such rows (1.26x) and
-// inflow lattices of 1000 MiB or more (1.01-1.17x).
-// By the rule 3283 of the 6279 shapes take two steps per pass, at 1.24x on
-// average; 34 of them are slower by more than 3 %, the slowest at 0.88 (before
-// there was the second line 1937 were, the slowest at 0.54).
+//    hold nodes as well, from where two steps per pass are the faster way on
+//    average over 6279 shapes of 15 MB to 4 GB (l 7 to 256, m : n from 1 : 4 to 4 : 1,
+//    32 to 64 steps through the captured graph, with and without a sphere).
+//    Below, the one-step sweep still finds part of its state in L2, and the
+//    two-step sweep has few blocks, whose slowest ends the launch: those at a wall
+//    or at an obstacle.
+// What the node line goes by, each with two steps per pass against one:
+//  * rows that end inside a 32-byte sector, whose partial writes cost the one-step
+//    sweep more often: FP32 driven 90-110 MiB 1.20 against 0.97 for whole sectors,
+//    FP64 periodic 1.16 against 1.0;
+//  * FP64 arithmetic, whose tiles are 16 nodes wide: rows that leave a quarter or
+//    more of the one-step sweep's 32 lanes idle but not of the tiles' (l to 16, 33
+//    to 48) gain earlier, 1.07 and more from 15 MiB;
+//  * an obstacle: FP32 driven whole sectors below 300 MiB 0.74-0.95, FP64 0.76-0.98;
+//    the fused collision loses less to it (channel 1.04-1.22 from 90 MiB);
+//  * FP32 storage with FP64 arithmetic: half of FP64's bytes for its instructions,
+//    so the rims' second computation costs more than a pass saves (whole sectors
+//    0.86-1.04 but for inflow, with a sphere 0.64-0.93).
+// By the rule 4.2 thousand of the shapes take two steps per pass, at 1.20x on
+// average; 230 are slower by more than 3 % (without the node line 1960 were, and
+// mixed precision with a sphere ran at 0.81x).
 constexpr size_t kNever = SIZE_MAX >> 20;
 size_t two_step_line(int bcase) { return bcase == BC_PERIODIC ? 120 : (bcase == BC_INFLOW ? 300 : 150); }
-size_t two_step_node_line(int kind, int bcase, int l, bool obstacle) {
-    //                          driven, periodic, channel, inflow
-    static const size_t f32[2][4] = {{120, 80, 75, 0}, {400, 160, 200, 0}};
-    static const size_t f64[2][4] = {{125, 100, 110, 0}, {400, 200, 300, 400}};
-    if (kind == K_F32) return f32[obstacle][bcase];
-    const bool idle = 4 * 16 * ((l + 15LL) / 16) <= 3 * 32 * ((l + 31LL) / 32);
-    if (kind == K_F64) {
-        const size_t early = obstacle ? 110 : 80;
-        return idle ? std::min(early, f64[obstacle][bcase]) : f64[obstacle][bcase];
+size_t two_step_node_line(const bgk_lattice_desc* d, bool obstacle) {
+    // [rows end inside a sector][driven, periodic, channel, inflow]
+    static const size_t f32_open[2][4] = {{110, 70, 75, 0}, {85, 60, 70, 0}};
+    static const size_t f32_solid[2][4] = {{300, 125, 150, 0}, {110, 90, 90, 0}};
+    static const size_t f32_solid_fused[2][4] = {{200, 100, 90, 0}, {110, 90, 90, 0}};
+    static const size_t f64_open[2][4] = {{105, 95, 90, 0}, {75, 75, 60, 0}};
+    static const size_t f64_solid[2][4] = {{250, 165, 175, 0}, {110, 105, 105, 0}};
+    static const size_t mixed[2][4] = {{kNever, 600, kNever, 400}, {115, 115, 115, 0}};
+    const int b = d->bcase, part = ((long long)d->l * elem_bytes(d->kind)) % 32 != 0 ? 1 : 0;
+    if (d->kind == K_F32) return (!obstacle ? f32_open : (d->fast ? f32_solid_fused : f32_solid))[part][b];
+    const bool idle = 4 * 16 * ((d->l + 15LL) / 16) <= 3 * 32 * ((d->l + 31LL) / 32);
+    if (d->kind == K_F64) {
+        if (obstacle) return idle ? std::min<size_t>(105, f64_solid[part][b]) : f64_solid[part][b];
+        return idle ? 0 : f64_open[part][b];
     }
     if (obstacle) return kNever;
-    return idle ? 60 : (bcase == BC_INFLOW ? 1000 : kNever);
+    return idle ? 60 : mixed[part][b];
 }
 bool two_steps_pay(const bgk_lattice_desc* d, bool obstacle) {
     const size_t row = ((size_t)d->l * elem_bytes(d->kind) + 127) / 128 * 128;
-    return (37 * row * (size_t)d->m * (size_t)d->n >> 20) >= two_step_node_line(d->kind, d->bcase, d->l, obstacle);
+    return (37 * row * (size_t)d->m * (size_t)d->n >> 20) >= two_step_node_line(d, obstacle);
 }
 
 // Bytes of one more array, the rest population's second one, which a lattice

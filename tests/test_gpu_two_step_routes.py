@@ -88,11 +88,12 @@ def test_batches_count_their_two_step_members():
 # neighbours differs in what the rule looks at
 LINES = [
     (0, "periodic", (20, 95, 95), False, False), (0, "periodic", (38, 95, 95), False, True),       # nodes fill L2 or not
-    (0, "driven", (128, 56, 56), False, False), (0, "driven", (128, 80, 80), False, True),
+    (0, "driven", (24, 105, 100), False, False), (0, "driven", (128, 80, 80), False, True),
+    (1, "driven", (96, 90, 90), False, False), (1, "driven", (100, 90, 80), False, True),           # rows end inside a sector
     (1, "driven", (128, 128, 128), True, False), (1, "driven", (128, 128, 128), False, True),      # obstacle
-    (1, "channel", (101, 131, 67), True, False), (1, "channel", (101, 170, 100), True, True),
-    (1, "periodic", (100, 100, 80), True, False), (1, "periodic", (100, 100, 120), True, True),
-    (0, "driven", (128, 90, 90), True, False), (0, "driven", (128, 128, 128), True, True),
+    (1, "channel", (104, 100, 78), True, False), (1, "channel", (101, 131, 67), True, True),
+    (1, "periodic", (104, 90, 70), True, False), (1, "periodic", (104, 100, 120), True, True),
+    (0, "driven", (128, 80, 80), True, False), (0, "driven", (128, 128, 128), True, True),
     (0, "driven", (34, 120, 120), True, True),                                                      # idle lanes
     (4, "periodic", (128, 128, 128), False, False), (4, "periodic", (40, 150, 110), False, True),   # mixed precision
     (4, "driven", (128, 200, 200), False, False), (4, "channel", (33, 140, 130), False, True),
